@@ -12,7 +12,7 @@ ROOT = os.path.dirname(HERE)
 LIB = os.path.join(CSRC, "libscphd_b200.so")
 CLI = os.path.join(CSRC, "scphd_calibrate")   # command-line driver (links LIB)
 SOURCES = ["scphd_filter.cu", "scphd_server.cu", "scphd_io.cpp"]
-DEPS = SOURCES + ["scphd_kernels.cuh", "scphd_device.cuh", "scphd_cli.cpp"]
+DEPS = SOURCES + ["scphd_kernels.cuh", "scphd_fit_f32.cuh", "scphd_device.cuh", "scphd_cli.cpp"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

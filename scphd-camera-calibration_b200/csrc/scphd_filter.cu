@@ -310,7 +310,7 @@ public:
         carve(a);
         CUDA_TRY(cudaMemsetAsync(p, 0, probe.used, stream));
         merge_smem = merge_smem_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32, true);
-        fit_smem = cloud_fit_smem_bytes<T>(prm.P);
+        fit_smem = fit_kernel_smem_bytes<T>(prm.P);
         // with the kernel's static shared memory (20 KB at most), within 227 KB per block:
         // every particles_per_feature up to 256 fits (FP64 at 256: 147 KB of sample rows)
         if (fit_smem > 200 * 1024)
@@ -409,11 +409,11 @@ public:
             const int fs = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fs];
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             if (fit_specialised<T>(prm))
-                k_cloud_fit<T, K, kFitP><<<N * split, 256, fit_smem, stream>>>(
+                k_cloud_fit<T, K, kFitP><<<N * split, kFitThreads<T>, fit_smem, stream>>>(
                     prm, b, cur, M, fixed, pending ? 1 : 0, pending_dt, pending_frame, sample_frame[cur], zs[0], zs[1],
                     zs[2], split);
             else
-                k_cloud_fit<T, K><<<N * split, 256, fit_smem, stream>>>(prm, b, cur, M, fixed, pending ? 1 : 0,
+                k_cloud_fit<T, K><<<N * split, kFitThreads<T>, fit_smem, stream>>>(prm, b, cur, M, fixed, pending ? 1 : 0,
                                                                         pending_dt, pending_frame, sample_frame[cur],
                                                                         zs[0], zs[1], zs[2], split);
             LAUNCHED();
@@ -1389,7 +1389,7 @@ template <typename T> struct Batch final : scphd_batch {
                 stage_off[first + i] = stage_total;
                 stage_total += 3 * (size_t)pr.Mcap;
                 merge_smem = std::max(merge_smem, merge_smem_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32, true));
-                fit_smem = std::max(fit_smem, cloud_fit_smem_bytes<T>(pr.P));
+                fit_smem = std::max(fit_smem, fit_kernel_smem_bytes<T>(pr.P));
                 fused_smem = std::max(fused_smem, fused_smem_bytes<T>(pr.P, pr.Gcap, pr.Scap));
                 lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block));
             }
@@ -1483,10 +1483,10 @@ template <typename T> struct Batch final : scphd_batch {
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             for (const Group& g : groups) {
                 if (g.fit_p)
-                    k_cloud_fit_batch<T, KK, kFitP><<<g.n_parent * split, 256, fit_smem, stream>>>(
+                    k_cloud_fit_batch<T, KK, kFitP><<<g.n_parent * split, kFitThreads<T>, fit_smem, stream>>>(
                         *g.tab, d_fa + g.first, g.map_parent, split);
                 else
-                    k_cloud_fit_batch<T, KK><<<g.n_parent * split, 256, fit_smem, stream>>>(*g.tab, d_fa + g.first,
+                    k_cloud_fit_batch<T, KK><<<g.n_parent * split, kFitThreads<T>, fit_smem, stream>>>(*g.tab, d_fa + g.first,
                                                                                             g.map_parent, split);
                 LAUNCHED();
             }

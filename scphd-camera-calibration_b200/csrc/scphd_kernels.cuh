@@ -614,29 +614,51 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
     }
 }
 
+}  // namespace scphd
+#include "scphd_fit_f32.cuh"
+namespace scphd {
+
+// the cloud fit's body by precision: four samples per lane in FP32, one in FP64
+template <typename T, int K, int PC>
+__device__ __forceinline__ void cloud_fit_any(const Params& prm, const Bufs<T>& b, int cur, int M, int fixed,
+                                              int has_pred, double dt, uint32_t pred_frame, uint32_t sample_frame,
+                                              const double* zu, const double* zv, const double* zd, int p, int c,
+                                              int split, unsigned char* smem) {
+    if constexpr (sizeof(T) == 4)
+        cloud_fit_f32_body<K, PC>(prm, b, cur, M, fixed, has_pred, dt, pred_frame, sample_frame, zu, zv, zd, p, c,
+                                    split, smem);
+    else
+        cloud_fit_body<T, K, PC>(prm, b, cur, M, fixed, has_pred, dt, pred_frame, sample_frame, zu, zv, zd, p, c,
+                                 split, reinterpret_cast<T*>(smem));
+}
+// threads of a cloud-fit block, and blocks an SM is to hold
+template <typename T> constexpr int kFitThreads = 32 * (sizeof(T) == 4 ? kQuadWarps : kFitWarps);
+template <typename T> constexpr int kFitBlocks = sizeof(T) == 4 ? 4 : 2;
+template <typename T> __host__ __device__ inline size_t fit_kernel_smem_bytes(int P) {
+    return sizeof(T) == 4 ? quad_fit_smem_bytes(P) : cloud_fit_smem_bytes<T>(P);
+}
 
 // grid: `split` blocks per parent (block x: parent x / split, part x % split)
 template <typename T, int K, int PC = 0>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
     k_cloud_fit(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int cur, int M, int fixed,
                 int has_pred, double dt, uint32_t pred_frame, uint32_t sample_frame, const double* zu,
                 const double* zv, const double* zd, int split) {
     extern __shared__ __align__(16) unsigned char dsm_fit[];
     const int p = blockIdx.x / split;
-    cloud_fit_body<T, K, PC>(prm, b, cur, M, fixed, has_pred, dt, pred_frame, sample_frame, zu, zv, zd, p,
-                             blockIdx.x - p * split, split, reinterpret_cast<T*>(dsm_fit));
+    cloud_fit_any<T, K, PC>(prm, b, cur, M, fixed, has_pred, dt, pred_frame, sample_frame, zu, zv, zd, p,
+                            blockIdx.x - p * split, split, dsm_fit);
 }
 
 template <typename T, int K, int PC = 0>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
     k_cloud_fit_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int split) {
     extern __shared__ __align__(16) unsigned char dsm_fit[];
     const int q = blockIdx.x / split;
     const int2 fp = map[q];
     const FrameArgs fa = fas[fp.x];
-    cloud_fit_body<T, K, PC>(tab.prm[fp.x], tab.b[fp.x], fa.cur, fa.M, fa.fixed, fa.has_pred, fa.dt, fa.pred_frame,
-                             fa.sample_frame, fa.zu, fa.zv, fa.zd, fp.y, blockIdx.x - q * split, split,
-                             reinterpret_cast<T*>(dsm_fit));
+    cloud_fit_any<T, K, PC>(tab.prm[fp.x], tab.b[fp.x], fa.cur, fa.M, fa.fixed, fa.has_pred, fa.dt, fa.pred_frame,
+                            fa.sample_frame, fa.zu, fa.zv, fa.zd, fp.y, blockIdx.x - q * split, split, dsm_fit);
 }
 
 // ---------------------------------------------------------------- (c0) Kalman terms
