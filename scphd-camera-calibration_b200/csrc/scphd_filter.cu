@@ -96,6 +96,7 @@ struct scphd_filter {
     // first updates that have measurements: threads per merge block, and whether the
     // likelihood runs one block over all of a parent's measurements or 128-thread blocks.
     // Each shape runs twice, the update is timed with events, the fastest is kept.
+    // Each merge width has its launch's survivor capacity (merge_launch_cap).
     struct Shape { int merge_threads; int lik_full; };
     static constexpr int kShapes = 4;
     const Shape shapes[kShapes] = {{kMergeThreads, 1}, {128, 1}, {kMergeThreads, 0}, {128, 0}};
@@ -241,7 +242,9 @@ public:
     Bufs<T> b{};
     void* arena_ptr = nullptr;
     T* dump = nullptr;        // Gcap x 7 x Ps cloud dump scratch
-    size_t merge_smem = 0;
+    size_t merge_smem = 0;       // the full survivor capacity's
+    int merge_over_grid = 0;     // blocks of the second merge launch
+    struct MergeLaunch { int S = 0; size_t smem = 0; } merge_at[2];   // first launch: kMergeThreads, 128 threads
     size_t fit_smem = 0;
 
     ~Filter() override {
@@ -309,15 +312,16 @@ public:
         a.cap = probe.used;
         carve(a);
         CUDA_TRY(cudaMemsetAsync(p, 0, probe.used, stream));
-        merge_smem = merge_smem_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32, true);
+        merge_smem = merge_shared_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32);
         fit_smem = fit_kernel_smem_bytes<T>(prm.P);
         // with the kernel's static shared memory (20 KB at most), within 227 KB per block:
         // every particles_per_feature up to 256 fits (FP64 at 256: 147 KB of sample rows)
         if (fit_smem > 200 * 1024)
             return fail(SCPHD_ERR_CAPACITY, "particles_per_feature needs " + std::to_string(fit_smem) +
                                                 " bytes of shared memory per cloud-fit block (limit 200 KB)");
-        if (merge_smem > 227 * 1024)
-            return fail(SCPHD_ERR_CAPACITY, "max_survivors/max_gaussians need " + std::to_string(merge_smem) +
+        const size_t merge_need = merge_smem_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32, true);
+        if (merge_need > 227 * 1024)
+            return fail(SCPHD_ERR_CAPACITY, "max_survivors/max_gaussians need " + std::to_string(merge_need) +
                                                 " bytes of shared memory per merge block (limit 227 KB)");
         const void* fused_fn = prm.K == 2 ? (const void*)k_fused<T, 2> : (const void*)k_fused<T, 3>;
         if (prm.K == 2) {
@@ -332,6 +336,20 @@ public:
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit<T, 3, kFitP>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 3>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_prep<T, 3>));
+        }
+        {
+            const void* merge_fn = prm.K == 2 ? (const void*)k_merge<T, 2> : (const void*)k_merge<T, 3>;
+            int dev = 0, nsm = 0, occ = 0;
+            CUDA_TRY(cudaGetDevice(&dev));
+            CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, merge_fn, kMergeThreads, merge_smem));
+            merge_over_grid = std::min(prm.N, nsm * occ);
+            // a filter whose parents are all resident at the full capacity takes one launch
+            for (int k = 0; k < 2; ++k) {
+                const int threads = k == 0 ? kMergeThreads : 128, blocks = kMergeBlocks<T> * (kMergeThreads / threads);
+                merge_at[k].S = prm.N <= merge_over_grid ? prm.Scap : merge_launch_cap<T>(prm.Scap, prm.Gcap, threads, blocks);
+                merge_at[k].smem = merge_shared_bytes<T>(merge_at[k].S, prm.Gcap, threads / 32);
+            }
         }
         fused_smem = fused_smem_bytes<T>(prm.P, prm.Gcap, prm.Scap);
         fused_grid = 0;
@@ -435,8 +453,13 @@ public:
                 stage_end(h);
             }
             h = stage_begin(3);
-            k_merge<T, K><<<N, sh.merge_threads, merge_smem, stream>>>(prm, b, cur, M, fixed);
+            const MergeLaunch& ml = merge_at[sh.merge_threads == kMergeThreads ? 0 : 1];
+            k_merge<T, K><<<N, sh.merge_threads, ml.smem, stream>>>(prm, b, cur, M, fixed, ml.S, 0);
             LAUNCHED();
+            if (ml.S < prm.Scap) {
+                k_merge<T, K><<<merge_over_grid, kMergeThreads, merge_smem, stream>>>(prm, b, cur, M, fixed, prm.Scap, 1);
+                LAUNCHED();
+            }
             stage_end(h);
         }
         pending = false;
@@ -1284,6 +1307,7 @@ template <typename T> struct Batch final : scphd_batch {
         int4* map_lik = nullptr;    int n_lik = 0;
         int* work = nullptr;            // the fused update's work counter
         bool fit_p = false;             // every member has kFitP samples per feature
+        int merge_over = 0;             // blocks per filter of the second merge launch (0: none needed)
     };
     int K = 3;
     bool use_graph = false;
@@ -1299,7 +1323,9 @@ template <typename T> struct Batch final : scphd_batch {
     double* d_stage = nullptr;
     std::vector<size_t> stage_off;
     size_t stage_total = 0;
-    size_t merge_smem = 0;
+    size_t merge_smem = 0;       // the members' full survivor capacities
+    size_t merge_first_smem = 0; // the first launch's (Params::Ssm)
+    size_t merge_need = 0;       // the limit's (merge_smem_bytes)
     size_t fit_smem = 0;
     size_t lik_smem = 0;
     int lik_block = 32;
@@ -1388,7 +1414,12 @@ template <typename T> struct Batch final : scphd_batch {
                     for (int k = 0; k < mb; ++k) ml.back().push_back(make_int4(i, q, k, 0));
                 stage_off[first + i] = stage_total;
                 stage_total += 3 * (size_t)pr.Mcap;
-                merge_smem = std::max(merge_smem, merge_smem_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32, true));
+                merge_need = std::max(merge_need, merge_smem_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32, true));
+                merge_smem = std::max(merge_smem, merge_shared_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
+                const int S = merge_launch_cap<T>(pr.Scap, pr.Gcap, kMergeThreads, kMergeBlocks<T>);
+                g.tab->prm[i].Ssm = S;
+                merge_first_smem = std::max(merge_first_smem, merge_shared_bytes<T>(S, pr.Gcap, kMergeThreads / 32));
+                if (S < pr.Scap) g.merge_over = std::max(g.merge_over, std::min(pr.N, 16));
                 fit_smem = std::max(fit_smem, fit_kernel_smem_bytes<T>(pr.P));
                 fused_smem = std::max(fused_smem, fused_smem_bytes<T>(pr.P, pr.Gcap, pr.Scap));
                 lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block));
@@ -1425,7 +1456,7 @@ template <typename T> struct Batch final : scphd_batch {
         }
         CUDA_TRY(cudaMallocHost(&h_fa, sizeof(FrameArgs) * F));
         CUDA_TRY(cudaMallocHost(&h_stage, sizeof(double) * std::max<size_t>(stage_total, 1)));
-        if (merge_smem > 227 * 1024) return fail(SCPHD_ERR_CAPACITY, "batch merge needs more than 227 KB of shared memory");
+        if (merge_need > 227 * 1024) return fail(SCPHD_ERR_CAPACITY, "batch merge needs more than 227 KB of shared memory");
         {
             const void* fn = K == 2 ? (const void*)k_fused_batch<T, 2> : (const void*)k_fused_batch<T, 3>;
             fused_grid = 0;
@@ -1505,7 +1536,14 @@ template <typename T> struct Batch final : scphd_batch {
             }
             const int mt = pth == 1 ? 128 : kMergeThreads;
             for (const Group& g : groups) {
-                k_merge_batch<T, KK><<<g.n_parent, mt, merge_smem, stream>>>(*g.tab, d_fa + g.first, g.map_parent);
+                k_merge_batch<T, KK><<<g.n_parent, mt, merge_first_smem, stream>>>(*g.tab, d_fa + g.first, g.map_parent,
+                                                                                   g.count, 0);
+                LAUNCHED();
+            }
+            for (const Group& g : groups) {
+                if (!g.merge_over) continue;
+                k_merge_batch<T, KK><<<g.count * g.merge_over, kMergeThreads, merge_smem, stream>>>(*g.tab, d_fa + g.first,
+                                                                                                   g.map_parent, g.count, 1);
                 LAUNCHED();
             }
         }
@@ -1524,7 +1562,11 @@ template <typename T> struct Batch final : scphd_batch {
         return SCPHD_OK;
     }
 
-    int launches_per_frame() const { return (path_now() == 2 ? 4 : 7) * (int)groups.size(); }
+    int launches_per_frame() const {
+        int n = 0;
+        for (const Group& g : groups) n += path_now() == 2 ? 4 : 7 + (g.merge_over > 0);
+        return n;
+    }
 
     scphd_status set_fused(int mode) override {
         if (mode < 0 || mode > 1) return fail(SCPHD_ERR_INVALID, "mode must be 0 or 1");

@@ -25,6 +25,7 @@ namespace scphd {
 
 struct Params {
     int N, P, Ps, Gcap, Mcap, Scap, K;
+    int Ssm;         // survivor capacity of a batch's first merge launch (merge_launch_cap)
     Model model;
     ModelF model_f;   // model's transform constants in FP32
     double kappa, ps, min_weight, min_sep, min_neff;
@@ -71,7 +72,7 @@ template <typename T> struct Bufs {
     double* loglik;     // N
     double* cum;        // N resampling prefix
     double* scal;       // [0] neff
-    int* flags;         // [0] resampled
+    int* flags;         // [0] resampled, [2] fused work counter, [3] parents listed for the second merge launch
     int* resample_idx;  // N
     unsigned long long* counters;   // 16
     int* fit_n;         // N: Gaussians the last update fitted (prior map size)
@@ -325,6 +326,7 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
     // the two poses (FP64 rotation terms) by threads of two warps, side by side
     if (threadIdx.x == 32) pose_src = make_pose<T>(b.map_ext[cur] + 12 * row);
     if (threadIdx.x == 0) {
+        if (p == 0 && c == 0) b.flags[3] = 0;   // no parent listed for a second merge launch yet
         double zero[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
         pose_upd = make_pose<T>(fixed ? zero : b.ext + 12 * p);
         if (c == 0) {
@@ -1281,6 +1283,7 @@ template <typename T> struct MergeScratch {
 
 constexpr int kSmallComp = 8;       // components up to this size are merged by one thread
 constexpr int kMergeThreads = 256;   // threads of a parent's merge block (8 warps)
+template <typename T> constexpr int kMergeBlocks = sizeof(T) == 4 ? 3 : 2;   // blocks per SM by registers
 
 __host__ __device__ inline int next_pow2(int x) {
     int p = 1;
@@ -1307,16 +1310,17 @@ template <typename T> inline size_t merge_smem_bytes(int S, int G, int nwarps, b
     return merge_stage_bytes<T>(S, stage) + cap * (sizeof(T) + 8) + (pf > pos ? pf : pos) + 3 * (size_t)S * 4 +
            cap * 4 + (size_t)(S + 1) * 4 + (size_t)nwarps * nchunk * 4 + 2 * (size_t)S + 64;
 }
+// shared memory of a caller's list of up to S components (merge_smem_bytes(S, 0, ., false))
 template <typename T>
-__device__ inline void carve_merge_smem(unsigned char* smem, int S, int G, bool stage, T*& s_w, uint32_t*& s_key,
+__device__ inline void carve_merge_list(unsigned char* smem, int S, T*& s_w, uint32_t*& s_key,
                                         int*& s_r, int*& s_pos, MergeScratch<T>& ms) {
-    const int cap = merge_sort_cap(S, G);
-    s_w = reinterpret_cast<T*>(smem + merge_stage_bytes<T>(S, stage));
+    const int cap = merge_sort_cap(S, 0);
+    s_w = reinterpret_cast<T*>(smem);
     s_key = reinterpret_cast<uint32_t*>(s_w + cap);
     s_r = reinterpret_cast<int*>(s_key + cap);
     ms.pf = reinterpret_cast<float*>(s_r + cap);
     s_pos = reinterpret_cast<int*>(ms.pf);   // positions are used only once the prefilter rows are dead
-    ms.lab = reinterpret_cast<int*>(ms.pf + (6 * S > S + G ? 6 * S : S + G));
+    ms.lab = reinterpret_cast<int*>(ms.pf + 6 * S);
     ms.cidx = ms.lab + S;
     ms.fill = ms.cidx + S;
     ms.perm = ms.fill + S;
@@ -1325,6 +1329,60 @@ __device__ inline void carve_merge_smem(unsigned char* smem, int S, int G, bool 
     ms.masks = reinterpret_cast<uint32_t*>(ms.start + S + 1);
     ms.flag = reinterpret_cast<uint8_t*>(ms.masks + (blockDim.x / 32) * ms.nchunk);
     ms.is_center = ms.flag + S;
+}
+
+// The filter's merge keeps less at a time than that: arrays that are never live together
+// share their bytes.  The means' area holds the sort keys before them and the new map's
+// weights after them, the ranks' holds the member lists, the u keys' the component indices,
+// the prefilter's the output positions.  (merge_smem_bytes stays the limit that scphd_create
+// and scphd_batch_create check.)
+template <typename T> __host__ __device__ inline size_t merge_area_bytes(int S, int G) {
+    const size_t stage = merge_stage_bytes<T>(S, true), keys = sizeof(T) == 4 ? 8 * (size_t)next_pow2(S) : 0;
+    const size_t out = (size_t)(S + G) * sizeof(T);
+    const size_t m = stage > keys ? (stage > out ? stage : out) : (keys > out ? keys : out);
+    return (m + 15) & ~(size_t)15;
+}
+template <typename T> __host__ __device__ inline size_t merge_shared_bytes(int S, int G, int nwarps) {
+    const size_t pad = next_pow2(S), pf = 6 * (size_t)S > (size_t)(S + G) ? 6 * (size_t)S : (size_t)(S + G);
+    return merge_area_bytes<T>(S, G) + pad * (sizeof(T) + 8) + 4 * (pf + 3 * (size_t)S + 1) +
+           (size_t)nwarps * ((S + 31) / 32) * 4 + 2 * (size_t)S;
+}
+template <typename T>
+__device__ inline void carve_merge_shared(unsigned char* smem, int S, int G, T*& s_w, uint32_t*& s_key, int*& s_r,
+                                          int*& s_pos, T*& s_out, MergeScratch<T>& ms) {
+    const int pad = next_pow2(S);
+    s_out = reinterpret_cast<T*>(smem);
+    s_w = reinterpret_cast<T*>(smem + merge_area_bytes<T>(S, G));
+    s_key = reinterpret_cast<uint32_t*>(s_w + pad);
+    s_r = reinterpret_cast<int*>(s_key + pad);
+    ms.pf = reinterpret_cast<float*>(s_r + pad);
+    s_pos = reinterpret_cast<int*>(ms.pf);
+    ms.lab = reinterpret_cast<int*>(ms.pf + (6 * S > S + G ? 6 * S : S + G));
+    ms.fill = ms.lab + S;
+    ms.start = ms.fill + S;
+    ms.cidx = reinterpret_cast<int*>(s_key);
+    ms.perm = s_r;
+    ms.nchunk = (S + 31) / 32;
+    ms.masks = reinterpret_cast<uint32_t*>(ms.start + S + 1);
+    ms.flag = reinterpret_cast<uint8_t*>(ms.masks + (blockDim.x / 32) * ms.nchunk);
+    ms.is_center = ms.flag + S;
+}
+
+// Survivor capacity of a merge launch.  Shared memory follows from it and so, where
+// max_survivors is far above what a parent has, do the blocks an SM holds: one at 1888
+// survivors (8192 parents x 512 Gaussians, which have about 570) and at 968 in FP64 (4096 x
+// 256, about 260), for a kernel that waits on barriers and dependent loads.  Where the full
+// capacity leaves an SM half the blocks that registers allow (`blocks`) or fewer, parents are
+// merged by a launch sized for `blocks`, and the few with more survivors, which it lists, by
+// a second one at the full capacity (4 us when the list is empty): 4.6 -> 2.8 ms and, in
+// FP64, 1.96 -> 1.32 ms at those sizes.  From two blocks to three there is nothing to gain
+// (FP32 at 968 survivors: 0.62 ms either way).
+template <typename T> inline int merge_launch_cap(int Scap, int G, int threads, int blocks) {
+    auto room = [](int n) { return (size_t)228 * 1024 / n - 1024 - 3584; };   // less what a block reserves, and static
+    if (merge_shared_bytes<T>(Scap, G, threads / 32) <= room(blocks / 2 + 1)) return Scap;
+    int S = 0;
+    while (S + 32 <= Scap && merge_shared_bytes<T>(S + 32, G, threads / 32) <= room(blocks)) S += 32;
+    return S >= G ? S : Scap;   // a parent seldom has fewer survivors than its map may hold
 }
 
 __device__ __forceinline__ bool could_merge_f(const float* a, const float* b, float min_sep, float margin) {
@@ -1736,20 +1794,27 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
     return s_stop;
 }
 
+// S: the launch's survivor capacity; a parent with more is listed for the second launch
+// (src_tmp, counted in flags[3], are free until the resampling) and left as it is
 template <typename T, int K>
-__device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, int cur, int M, int fixed, int p) {
+__device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, int cur, int M, int fixed, int p, int S) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x;
     const int G = min(b.map_n[cur][b.src[p]], prm.Gcap);
     const int n_all_surv = b.surv_n[p];
     const int n = min(n_all_surv, prm.Scap);
+    if (n > S) {
+        if (tid == 0) b.src_tmp[atomicAdd(b.flags + 3, 1)] = p;
+        return;
+    }
     const int n_pad = next_pow2(n);
     T* s_w;
     uint32_t* s_key;
     int* s_r;
     int* s_pos;
+    T* s_out;
     MergeScratch<T> ms;
-    carve_merge_smem<T>(smem, prm.Scap, prm.Gcap, true, s_w, s_key, s_r, s_pos, ms);
+    carve_merge_shared<T>(smem, S, prm.Gcap, s_w, s_key, s_r, s_pos, s_out, ms);
     __shared__ int s_tmp[40];
     // FP32: packed sort keys in the survivor staging area (free until the survivors are
     // staged; 8 n_pad <= 16 Scap bytes fit in its 28 Scap); FP64: (weight, tie key, rank)
@@ -1821,7 +1886,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     KalmanView<T> view;
     {
         T* st_mu = reinterpret_cast<T*>(smem);
-        T* st_bcov = st_mu + 6 * prm.Scap;
+        T* st_bcov = st_mu + 6 * S;
         int* st_cj = reinterpret_cast<int*>(st_bcov + 21);
         for (int i = tid; i < n; i += blockDim.x) {
             const int r = s_r[i];
@@ -1865,7 +1930,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
             const T wnd = nd_weight(fr[0], fr[1]);
             w = (wnd >= minw) ? wnd : T(-1);   // -1: not retained
         }
-        s_w[e] = w;
+        s_out[e] = w;
         n_valid_part += w >= T(0);
     }
     __shared__ int s_nvalid;
@@ -1876,14 +1941,14 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     const bool cut = s_nvalid > prm.Gcap;
     // keep: retained, and when over capacity among the Gcap largest (ties by entry order)
     if (!cut) {
-        for (int e = tid; e < n_all; e += blockDim.x) s_pos[e] = s_w[e] >= T(0);
+        for (int e = tid; e < n_all; e += blockDim.x) s_pos[e] = s_out[e] >= T(0);
         __syncthreads();
     } else {
-        const uint64_t thr = select_kth_largest(s_w, n_all, prm.Gcap);
+        const uint64_t thr = select_kth_largest(s_out, n_all, prm.Gcap);
         // entries above the threshold, then ties in entry order up to Gcap
         int above = 0;
         for (int e = tid; e < n_all; e += blockDim.x) {
-            const T w = s_w[e];
+            const T w = s_out[e];
             const uint64_t key = w >= T(0) ? weight_key(w) : 0ull;
             above += key > thr;
             s_pos[e] = (w >= T(0) && key == thr) ? 1 : 0;
@@ -1896,7 +1961,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
         const int ties_keep = prm.Gcap - s_above;
         block_exclusive_scan(s_pos, n_all, s_tmp);   // rank among the ties
         for (int e = tid; e < n_all; e += blockDim.x) {
-            const T w = s_w[e];
+            const T w = s_out[e];
             const uint64_t key = w >= T(0) ? weight_key(w) : 0ull;
             const bool tie = w >= T(0) && key == thr;
             s_pos[e] = (w >= T(0) && key > thr) || (tie && s_pos[e] < ties_keep);
@@ -1922,7 +1987,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
             mr[pos] = -1 - e;
         } else {
             const int j = e - n_out;
-            mo[(size_t)pos * kRow] = s_w[e];
+            mo[(size_t)pos * kRow] = s_out[e];
             mr[pos] = p * prm.Gcap + j;
         }
     }
@@ -1941,18 +2006,32 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     }
 }
 
+// over = 0: block p merges parent p, survivor capacity S; over = 1: the listed parents, at
+// the full capacity, dealt out over the blocks
 template <typename T, int K>
-__global__ void __launch_bounds__(kMergeThreads, sizeof(T) == 4 ? 3 : 2) k_merge(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b,
-                                               int cur, int M, int fixed) {
-    merge_body<T, K>(prm, b, cur, M, fixed, blockIdx.x);
+__global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
+    k_merge(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int cur, int M, int fixed, int S, int over) {
+    const int n = over ? min(b.flags[3], prm.N) : prm.N;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        merge_body<T, K>(prm, b, cur, M, fixed, over ? b.src_tmp[i] : i, S);
+        __syncthreads();
+    }
 }
 
+// over = 0: a block per (filter, parent) of the map; over = 1: blockIdx.x % count is the
+// filter, its listed parents are dealt out over that filter's blocks
 template <typename T, int K>
-__global__ void __launch_bounds__(kMergeThreads, sizeof(T) == 4 ? 3 : 2)
-    k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map) {
-    const int2 fp = map[blockIdx.x];
+__global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
+    k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int over) {
+    const int2 fp = over ? make_int2(blockIdx.x % count, blockIdx.x / count) : map[blockIdx.x];
+    const Params& prm = tab.prm[fp.x];
+    const Bufs<T>& b = tab.b[fp.x];
     const FrameArgs fa = fas[fp.x];
-    merge_body<T, K>(tab.prm[fp.x], tab.b[fp.x], fa.cur, fa.M, fa.fixed, fp.y);
+    const int n = over ? min(b.flags[3], prm.N) : fp.y + 1, step = over ? gridDim.x / count : 1;
+    for (int i = fp.y; i < n; i += step) {
+        merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, over ? b.src_tmp[i] : i, over ? prm.Scap : prm.Ssm);
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------- fused update
@@ -1970,7 +2049,7 @@ constexpr int kFusedThreads = 256;
 template <typename T> inline size_t fused_smem_bytes(int P, int Gcap, int Scap) {
     size_t s = cloud_fit_smem_bytes<T>(P);
     const size_t cand[3] = {prep_smem_bytes<T>(), likelihood_smem_bytes<T>(Gcap, kFusedThreads),
-                            merge_smem_bytes<T>(Scap, Gcap, kFusedThreads / 32, true)};
+                            merge_shared_bytes<T>(Scap, Gcap, kFusedThreads / 32)};
     for (size_t c : cand) s = c > s ? c : s;
     return s;
 }
@@ -1986,7 +2065,7 @@ __device__ __forceinline__ void fused_parent(const Params& prm, const Bufs<T>& b
         likelihood_body<T, K>(prm, b, fa.cur, fa.M, p, mb, reinterpret_cast<T*>(smem));
         __syncthreads();
     }
-    merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, p);
+    merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, p, prm.Scap);
     __syncthreads();
 }
 
@@ -2386,7 +2465,7 @@ __global__ void __launch_bounds__(128) k_merge_list(const T* rows, const uint8_t
     int* s_r;
     int* s_pos;
     MergeScratch<T> ms;
-    carve_merge_smem<T>(smem, n_all + 1, 0, false, s_w, s_key, s_r, s_pos, ms);
+    carve_merge_list<T>(smem, n_all + 1, s_w, s_key, s_r, s_pos, ms);
     if (threadIdx.x == 0) {
         int k = 0;
         for (int i = 0; i < n_all; ++i)
