@@ -387,8 +387,8 @@ def run_b200(args):
         # map entries (merged component: 28 values; carried cloud: weight) read, fitted
         # rows (29) written, carried clouds read and candidate clouds written (7 P each)
         "cloud_fit": fitted * (28 + 29) * sz + (rd + wr) * 7 * P * sz,
-        # fitted rows (29) read, Kalman-term rows (48) and likelihood rows (12) written
-        "kalman_terms": fitted * (29 + 48 + 12) * sz,
+        # fitted rows (29) read, Kalman-term rows (44), weights (2) and likelihood rows (12) written
+        "kalman_terms": fitted * (29 + 44 + 2 + 12) * sz,
         # likelihood rows (12) read, normalisers written, survivors (rank + weight) written
         "likelihood": fitted * 12 * sz + ell_vals * sz + surv * (4 + sz),
         # survivors read with their Gaussians' gain, posterior covariance and fitted mean

@@ -282,8 +282,9 @@ scphd_status scphd_device_bytes(const scphd_config* cfg, int64_t* bytes);
 /* ------------------------------------------------------------------ batches
  * Many filters advanced together: every batched step runs predict(dt) + update +
  * resample for all member filters with one kernel launch per stage (seven per frame,
- * or four with the fused update, whatever the number of filters), each launch covering
- * every filter's parents
+ * or four with the fused update, whatever the number of filters; one more where
+ * max_survivors is large, for the parents with more survivors than most), each launch
+ * covering every filter's parents
  * through a block -> (filter, parent) map.  Member filters must share device,
  * precision and meas_dim; they may differ in size.  While in a batch, the filters
  * issue all their work on the batch's stream (their own stream is restored by

@@ -6,10 +6,9 @@
 //     a >= b, at a*(a+1)/2 + b (21 values);
 //   * a mixture component row is 32 T: [0] weight, [1..6] mean, [7..27] packed cov;
 //   * a fitted row is 32 T: [0] weight, [1] mean pD, [2..7] mean, [8..28] packed cov;
-//   * a prep row (per fitted Gaussian, measurement-independent Kalman terms) is
-//     48 T: [0] log-constant c, [1] PD flag of the posterior cov, [2..7] packed
-//     S^-1 (k x k, packed lower), [8..25] gain K (6 x 3, row-major), [26..46]
-//     packed posterior covariance.
+//   * a prep row (what the merge reads of a fitted Gaussian's Kalman terms) is 44 T:
+//     [0..17] gain K (6 x 3, row-major), [20..40] packed posterior covariance, both
+//     starting on 16 bytes.
 #pragma once
 
 #include <cstdint>
@@ -19,8 +18,8 @@
 namespace scphd {
 
 constexpr int kRow = 32;
-constexpr int kPrep = 48;
-constexpr int kPrepSi = 2, kPrepK = 8, kPrepCov = 26;
+constexpr int kPrep = 44;
+constexpr int kPrepK = 0, kPrepCov = 20;
 constexpr int kMaxLanesSamples = 8;   // particles_per_feature <= 256
 
 enum Stage : uint32_t { ST_PRIOR = 1, ST_CAM = 2, ST_FEAT = 3, ST_SAMPLE = 4, ST_RESAMPLE = 5 };
@@ -490,12 +489,11 @@ __device__ inline float mahal6<float>(const float* ma, const float* Sa, const fl
 // the gain K = P H' S^-1 and the Joseph-form posterior covariance
 // P - K(HP) - (HP)'K' + K(HPH')K' + K R K' (src/kernels.cu:506-595), then the
 // posterior's PD test (isPosDef, src/device_math.cu:800-812).  P is the fitted
-// packed covariance, Pn scratch for the posterior (21 values); dst receives [0]
-// log-constant, [1] PD flag, [2..7] S^-1 packed, [8..25] K (6 x 3 row-major),
-// [26..46] posterior covariance packed.
+// packed covariance, Pn scratch for the posterior (21 values); dst receives the prep row
+// (gain and posterior), cst the log-constant, Si the packed S^-1; returns the PD flag.
 template <typename T, int K>
-__device__ inline void kalman_prep(T w, T pdbar, const T* P, const Model& m, T* Pn, T* dst) {
-    T S[6], Si[6];
+__device__ inline bool kalman_prep(T w, T pdbar, const T* P, const Model& m, T* Pn, T* dst, T& cst, T (&Si)[6]) {
+    T S[6];
     S[0] = P[0] + (T)m.var[0];
     S[1] = P[1];
     S[2] = P[2] + (T)m.var[1];
@@ -516,7 +514,6 @@ __device__ inline void kalman_prep(T w, T pdbar, const T* P, const Model& m, T* 
         Si[3] = div_by(A20, det, idet); Si[4] = div_by(A21, det, idet); Si[5] = div_by(A22, det, idet);
     }
     const T log2pi = (T)1.8378770664093454835606594728112;
-    T cst;
     if (pdbar > T(0) && w > T(0) && det > T(0))
         cst = tlog(pdbar) + tlog(w) - T(0.5) * T(K) * log2pi - T(0.5) * tlog(det);
     else
@@ -566,11 +563,28 @@ __device__ inline void kalman_prep(T w, T pdbar, const T* P, const Model& m, T* 
         Pn[e] = sv;
         dst[kPrepCov + e] = sv;
     }
-    const bool pdok = posterior_pd(Pn);
-    dst[0] = cst;
-    dst[1] = pdok ? T(1) : T(0);
+    return posterior_pd(Pn);
+}
+
+// 16-byte pieces of N leading values of a row that starts on 16 bytes (and the values left
+// over), in plain loads: the fused update reads rows its own block wrote
+template <int N> __device__ __forceinline__ void load_head(const float* src, float* v) {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) dst[kPrepSi + q] = Si[q];
+    for (int i = 0; i < N / 4; ++i) {
+        const float4 x = reinterpret_cast<const float4*>(src)[i];
+        v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+    }
+#pragma unroll
+    for (int i = N / 4 * 4; i < N; ++i) v[i] = src[i];
+}
+template <int N> __device__ __forceinline__ void load_head(const double* src, double* v) {
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const double2 x = reinterpret_cast<const double2*>(src)[i];
+        v[2 * i] = x.x; v[2 * i + 1] = x.y;
+    }
+#pragma unroll
+    for (int i = N / 2 * 2; i < N; ++i) v[i] = src[i];
 }
 
 // log-likelihood exponent term c - 1/2 nu' S^-1 nu for measurement z

@@ -271,6 +271,8 @@ public:
         }
         b.fit = a.take<T>(N * G * kRow);
         b.prep = a.take<T>(N * G * kPrep);
+        b.birth = a.take<T>(kPrep);
+        b.wts = a.take<T>(N * G * 2);
         b.lik = a.take<T>(N * G * kLikTerms);
         b.z = a.take<T>(Mc * 3);
         b.ell = a.take<T>(N * Mc);
@@ -319,7 +321,7 @@ public:
         if (fit_smem > 200 * 1024)
             return fail(SCPHD_ERR_CAPACITY, "particles_per_feature needs " + std::to_string(fit_smem) +
                                                 " bytes of shared memory per cloud-fit block (limit 200 KB)");
-        const size_t merge_need = merge_smem_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32, true);
+        const size_t merge_need = merge_limit_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32);
         if (merge_need > 227 * 1024)
             return fail(SCPHD_ERR_CAPACITY, "max_survivors/max_gaussians need " + std::to_string(merge_need) +
                                                 " bytes of shared memory per merge block (limit 227 KB)");
@@ -362,6 +364,13 @@ public:
             fused_grid = std::min(prm.N, nsm * occ);
         }
         const int N = prm.N;
+        {   // the birth covariance, read like a posterior's
+            T row[kPrep] = {};
+            const double var[6] = {prm.model.var[0], prm.model.var[1], prm.K == 3 ? prm.model.var[2] : prm.var_d0,
+                                   prm.var_vu0, prm.var_vv0, prm.var_vd0};
+            for (int a2 = 0; a2 < 6; ++a2) row[kPrepCov + tri(a2, a2)] = (T)var[a2];
+            CUDA_TRY(cudaMemcpyAsync(b.birth, row, sizeof(row), cudaMemcpyHostToDevice, stream));
+        }
         k_prior<<<(N + 255) / 256, 256, 0, stream>>>(prm, b.ext, b.lw);
         LAUNCHED();
         k_iota<<<(N + 255) / 256, 256, 0, stream>>>(b.src, N);
@@ -1052,7 +1061,7 @@ scphd_status scphd_merge_components(const double* comps, const uint8_t* flags, i
         uint8_t* d_flags = nullptr;
         int* d_n = nullptr;
         int* d_mem = nullptr;
-        size_t smem = merge_smem_bytes<T>(n + 1, 0, 4, false);
+        size_t smem = merge_list_bytes<T>(n + 1, 4);
         T* d_sparse = nullptr;
         scphd_status st = SCPHD_OK;
         std::vector<T> out((size_t)n * kRow);
@@ -1181,7 +1190,7 @@ scphd_status merge_static_impl(unsigned char* base, const double* comps, const u
     CUDA_TRY(cudaMemset(d_mem, 0xff, sizeof(int) * (size_t)n));
     k_rows_from28<T><<<(n * kRow + 255) / 256, 256>>>(d_in, n, d_rows);
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    const size_t smem = merge_smem_bytes<T>(n + 1, 0, 4, false);
+    const size_t smem = merge_list_bytes<T>(n + 1, 4);
     CUDA_TRY(allow_dynamic_smem((const void*)k_merge_list<T>));
     k_merge_list<T><<<1, 128, smem>>>(d_rows, d_flags, n, (T)min_separation, d_sparse, d_out, d_cnt, d_mem);
     g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -1325,7 +1334,7 @@ template <typename T> struct Batch final : scphd_batch {
     size_t stage_total = 0;
     size_t merge_smem = 0;       // the members' full survivor capacities
     size_t merge_first_smem = 0; // the first launch's (Params::Ssm)
-    size_t merge_need = 0;       // the limit's (merge_smem_bytes)
+    size_t merge_need = 0;       // the limit's (merge_limit_bytes)
     size_t fit_smem = 0;
     size_t lik_smem = 0;
     int lik_block = 32;
@@ -1414,7 +1423,7 @@ template <typename T> struct Batch final : scphd_batch {
                     for (int k = 0; k < mb; ++k) ml.back().push_back(make_int4(i, q, k, 0));
                 stage_off[first + i] = stage_total;
                 stage_total += 3 * (size_t)pr.Mcap;
-                merge_need = std::max(merge_need, merge_smem_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32, true));
+                merge_need = std::max(merge_need, merge_limit_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
                 merge_smem = std::max(merge_smem, merge_shared_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
                 const int S = merge_launch_cap<T>(pr.Scap, pr.Gcap, kMergeThreads, kMergeBlocks<T>);
                 g.tab->prm[i].Ssm = S;

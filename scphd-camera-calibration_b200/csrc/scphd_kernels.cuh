@@ -60,6 +60,8 @@ template <typename T> struct Bufs {
     T* cloud[2];        // N*Gcap clouds of 7 x Ps (x,y,z,vx,vy,vz,omega)
     T* fit;             // N*Gcap rows of kRow
     T* prep;            // N*Gcap rows of kPrep (gain and posterior, read by the merge)
+    T* birth;           // a prep row with the birth covariance
+    T* wts;             // N*Gcap pairs: fitted weight, non-detection weight (-1: pruned)
     T* lik;             // N*Gcap rows of kLikTerms (the likelihood's per-Gaussian terms)
     T* z;               // Mcap x 3 measurements
     T* ell;             // N x Mcap normalisers
@@ -671,7 +673,8 @@ __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
 // other's latency).  Each thread reads its fitted row in 16-byte pieces and writes its
 // rows into shared memory (odd strides: no bank conflicts); the block then copies the
 // rows of its Gaussians -- contiguous in global memory -- out with coalesced stores:
-//   prep row (kPrep): the gain and posterior covariance the merge reads per survivor;
+//   prep row (kPrep): the gain and posterior covariance the merge reads per survivor, each
+//   from a 16-byte boundary;
 //   likelihood row (kLikTerms): log-constant (-inf when the posterior is not PD), PD
 //   flag, packed S^-1, mean (u, v, d) -- the k_likelihood terms, read in 16-byte pieces;
 //   in FP32 in base 2 (log2(e) c, S^-1 scaled for log2_term).
@@ -711,17 +714,22 @@ __device__ __forceinline__ void prep_body(const Params& prm, const Bufs<T>& b, i
         if ((int)threadIdx.x < n) {
             T v[29];
             load_row29(b.fit + ((size_t)p * prm.Gcap + j0 + threadIdx.x) * kRow, v);
-            T Pn[21];
+            T Pn[21], cst, Si[6];
             T* d = s_prep + (size_t)threadIdx.x * kPrepStride;
-            kalman_prep<T, K>(v[0], v[1], v + 8, prm.model, Pn, d);
-            d[kPrep - 1] = T(0);
+            const bool pd = kalman_prep<T, K>(v[0], v[1], v + 8, prm.model, Pn, d, cst, Si);
+            d[18] = d[19] = d[41] = d[42] = d[43] = T(0);
+            // what the merge needs of the weight: the fitted one, and the non-detection term's
+            const T wnd = nd_weight(v[0], v[1]);
+            T* gw = b.wts + ((size_t)p * prm.Gcap + j0 + threadIdx.x) * 2;
+            gw[0] = v[0];
+            gw[1] = wnd >= (T)prm.min_weight ? wnd : T(-1);
             T* l = s_lik + (size_t)threadIdx.x * kLikStride;
             // a non-PD posterior's log-constant is staged as -inf (its weight is LOG0 before
             // the normaliser, kernels.cu:597-598), so the normaliser pass needs no test
-            l[0] = (d[0] > tneg_inf<T>() && d[1] != T(0)) ? d[0] : tneg_inf<T>();
-            l[1] = d[1];
+            l[0] = (cst > tneg_inf<T>() && pd) ? cst : tneg_inf<T>();
+            l[1] = pd ? T(1) : T(0);
 #pragma unroll
-            for (int i = 0; i < 6; ++i) l[2 + i] = d[kPrepSi + i];
+            for (int i = 0; i < 6; ++i) l[2 + i] = Si[i];
             if constexpr (sizeof(T) == 4) {   // base-2 form (log2_term): c2 and the scaled S^-1
                 l[0] = l[0] * kLog2e;
 #pragma unroll
@@ -977,25 +985,25 @@ __global__ void __launch_bounds__(1024)
 // ---------------------------------------------------------------- (d) merge
 // Posterior components of one parent (detections and births) by survivor rank r: the
 // mean, from the fitted row, the Kalman gain and the measurement (a birth's from the
-// birth template); bcov holds the birth covariance, the detections' covariances are
-// their Gaussians' posteriors in the prep rows.
+// birth template); the covariances are their Gaussians' posteriors in the prep rows, or
+// the birth row's.
 template <typename T, int K> struct KalmanSource {
     const T* fit;   // parent's fitted rows
     const T* prep;  // parent's prep rows
     const T* z;     // measurements
     int G, M;
-    T bmean[6], bcov[21];   // birth template (mean[0..K) replaced by z)
+    T bmean[6];     // birth template (mean[0..K) replaced by z)
     __device__ void mean(int r, T mu[6]) const {
         if (r < G * M) {
             int mm = r / G, j = r - mm * G;
-            const T* fr = fit + (size_t)j * kRow;
-            const T* Kg = prep + (size_t)j * kPrep + kPrepK;
-            T nu[3];
+            T fm[8], Kg[18], nu[3];
+            load_head<8>(fit + (size_t)j * kRow, fm);
+            load_head<18>(prep + (size_t)j * kPrep + kPrepK, Kg);
 #pragma unroll
-            for (int a = 0; a < K; ++a) nu[a] = z[mm * 3 + a] - fr[2 + a];
+            for (int a = 0; a < K; ++a) nu[a] = z[mm * 3 + a] - fm[2 + a];
 #pragma unroll
             for (int a = 0; a < 6; ++a) {
-                T s = fr[2 + a];
+                T s = fm[2 + a];
 #pragma unroll
                 for (int c = 0; c < K; ++c) s += nu[c] * Kg[a * 3 + c];
                 mu[a] = s;
@@ -1017,31 +1025,47 @@ template <typename T, int K> struct KalmanSource {
 // parent's prep rows.
 template <typename T> struct ListView {
     static constexpr bool kSelfAbsorbs = false;   // caller's rows: the self-distance is evaluated
+    static constexpr bool kScansPairs = false, kFloatMeans = false;
     const T* rows;
     const int* s_r;
+    __device__ const float* float_means(const float* copies) const { return copies; }
     __device__ void mean(int i, T mu[6]) const {
         const T* r = rows + (size_t)s_r[i] * kRow + 1;
 #pragma unroll
         for (int a = 0; a < 6; ++a) mu[a] = r[a];
     }
     __device__ const T* cov(int i) const { return rows + (size_t)s_r[i] * kRow + 7; }
+    __device__ void cov(int i, T (&c)[21]) const {
+        const T* p = cov(i);
+#pragma unroll
+        for (int e = 0; e < 21; ++e) c[e] = p[e];
+    }
 };
 template <typename T> struct KalmanView {
     // every component has a PD covariance (posteriors passed the PD test, births are
     // diagonal), so a centre's distance to itself is exactly 0 < min_separation
     static constexpr bool kSelfAbsorbs = true;
-    const T* mu;      // S x 6
+    static constexpr bool kScansPairs = true, kFloatMeans = sizeof(T) == 4;
+    const T* mu;      // 6 x S
+    int S;
     const int* cj;    // S
     const T* covs;    // Gaussian j's covariance at covs + j * kPrep
-    const T* bcov;    // birth covariance (21, shared memory)
+    const T* bcov;    // birth covariance
     __device__ void mean(int i, T m[6]) const {
 #pragma unroll
-        for (int a = 0; a < 6; ++a) m[a] = mu[i * 6 + a];
+        for (int a = 0; a < 6; ++a) m[a] = mu[a * S + i];
+    }
+    __device__ const float* float_means(const float* copies) const {
+        if constexpr (kFloatMeans) return mu;
+        else return copies;
     }
     __device__ const T* cov(int i) const {
         const int j = cj[i];
         return j >= 0 ? covs + (size_t)j * kPrep : bcov;
     }
+    // in 16-byte pieces: lanes read different rows, so a scalar load costs as many
+    // cache-line accesses as a wide one
+    __device__ void cov(int i, T (&c)[21]) const { load_head<21>(cov(i), c); }
 };
 
 // Order of the greedy merge's argmax (and of the map-capacity cut): by weight rounded
@@ -1057,160 +1081,123 @@ template <typename T> __device__ __forceinline__ bool merge_before(T wa, uint32_
     return fa > fb || (fa == fb && ka < kb);
 }
 
-// Bitonic sort of n_pad (a power of two) items in shared arrays, ordered by
-// Items::before.  The comparator network is the textbook one (for k = 2, 4, ..:
-// for j = k/2 .. 1: items i and i^j swap when the later should come first, in the
-// direction of bit k of i).  When the block splits the items into one chunk of 32 R
-// items per warp (R = 1..8), every stage whose partners lie in the same chunk runs in
-// registers (j < 32: shuffles across lanes; 32 <= j < 32 R: within a thread), and only
-// the stages with j >= 32 R go through shared memory, each behind a barrier; otherwise
-// every stage does.  Both give the network's result.  Starts and ends with a barrier.
-template <typename T> struct SurvItems {   // (weight, tie key, rank) by merge_before
-    T* w;
-    uint32_t* key;
-    int* r;
-    struct Item { T w; uint32_t key; int r; };
-    __device__ Item load(int i) const { return Item{w[i], key[i], r[i]}; }
-    __device__ void store(int i, const Item& x) const { w[i] = x.w; key[i] = x.key; r[i] = x.r; }
-    __device__ static bool before(const Item& a, const Item& b) { return merge_before(a.w, a.key, b.w, b.key); }
-    __device__ static Item shfl(const Item& x, int m) {
-        return Item{__shfl_xor_sync(0xffffffffu, x.w, m), __shfl_xor_sync(0xffffffffu, x.key, m),
-                    __shfl_xor_sync(0xffffffffu, x.r, m)};
-    }
-};
-struct KeyItems {   // (key, value) by ascending key
-    uint32_t* key;
-    int* val;
-    struct Item { uint32_t key; int val; };
-    __device__ Item load(int i) const { return Item{key[i], val[i]}; }
-    __device__ void store(int i, const Item& x) const { key[i] = x.key; val[i] = x.val; }
-    __device__ static bool before(const Item& a, const Item& b) { return a.key < b.key; }
-    __device__ static Item shfl(const Item& x, int m) {
-        return Item{__shfl_xor_sync(0xffffffffu, x.key, m), __shfl_xor_sync(0xffffffffu, x.val, m)};
-    }
-};
-
-// FP32 survivors as one 64-bit key each, sorted descending: the weight's bits (a
-// non-negative float orders as its bit pattern) above the complement of the tie key,
-// so that the order is merge_before's; padding slots hold 0 and sort last.  Half the
-// shuffles and a single compare per exchange against SurvItems.
-struct PackedSurvItems {
-    unsigned long long* k;
-    typedef unsigned long long Item;
-    __device__ Item load(int i) const { return k[i]; }
-    __device__ void store(int i, const Item& x) const { k[i] = x; }
-    __device__ static bool before(const Item& a, const Item& b) { return a > b; }
-    __device__ static Item shfl(const Item& x, int m) { return __shfl_xor_sync(0xffffffffu, x, m); }
-};
+// A survivor's sort key: the order key's bits, made to order as the float (and the two zeros
+// as one), above the complement of the tie key, so that larger keys come first by
+// merge_before, every key is distinct and none is 0 (the padding).
+__device__ __forceinline__ uint32_t float_order(float x) {
+    const uint32_t bits = __float_as_uint(x + 0.0f);
+    return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
+}
 __device__ __forceinline__ unsigned long long pack_survivor(float w, uint32_t r) {
-    return ((unsigned long long)__float_as_uint(w) << 32) | (uint32_t)~tie_key(r);
-}
-__device__ __forceinline__ uint32_t untie_key(uint32_t t) {   // inverse of tie_key
-    return ((t & 0xffffffu) << 8) | (__brev(t >> 24) >> 24);
+    return ((unsigned long long)float_order(w) << 32) | (uint32_t)~tie_key(r);
 }
 
-// one shared-memory stage (k, j) over all pairs
-template <typename Items>
-__device__ __forceinline__ void bitonic_smem_stage(const Items& it, int n_pad, int k, int jj) {
-    for (int i = threadIdx.x; i < n_pad; i += blockDim.x) {
-        const int ixj = i ^ jj;
-        if (ixj > i) {
-            const bool up = (i & k) == 0;
-            const typename Items::Item lo = it.load(i), hi = it.load(ixj);
-            if (Items::before(hi, lo) == up) {
-                it.store(i, hi);
-                it.store(ixj, lo);
-            }
-        }
-    }
-}
-
-// stage (k, j) with 32 <= j < 32 R: pairs (r, r | D) of one thread, D = j / 32
-template <int R, int D, typename Items>
-__device__ __forceinline__ void bitonic_thread_stage(typename Items::Item (&x)[R], int base, int lane, int k) {
+// Bitonic sort, larger keys first, of n_pad (a power of two) 64-bit keys in shared memory;
+// they are distinct but for padding zeros.  The comparator network is the textbook one (for
+// k = 2, 4, ..: for j = k/2 .. 1: items i and i^j, in the direction of bit k of i).  Each warp
+// holds a chunk of 32 R items in registers (R = 1..8; item base + 32 r + lane), where the
+// stages with j < 32 R run: j < 32 by shuffles, 32 <= j within a thread.  Items that a k runs
+// in the other direction are complemented for its stages, so that a stage needs one
+// comparison and no direction.  Only the stages with j >= 32 R go through shared memory, each
+// behind a barrier.  (Before: a key and its index or three words, a direction per item and
+// stage and loops over j; 18k of a merge's 47k warp instructions at 253 survivors.)
+// Starts and ends with a barrier.
+template <int R, int J> __device__ __forceinline__ void sort64_stage(unsigned long long (&x)[R], int lane) {
+    if constexpr (J >= 32) {
+        constexpr int D = J / 32;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        if ((r & D) == 0 && (r | D) < R) {
-            const bool up = ((base + r * 32 + lane) & k) == 0;
-            if (Items::before(x[r | D], x[r]) == up) {
-                const typename Items::Item t = x[r];
+        for (int r = 0; r < R; ++r)
+            if ((r & D) == 0 && (r | D) < R && x[r | D] > x[r]) {
+                const unsigned long long t = x[r];
                 x[r] = x[r | D];
                 x[r | D] = t;
             }
+    } else {
+        const bool lower = (lane & J) == 0;   // the lower item keeps the larger key
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const unsigned long long q = __shfl_xor_sync(0xffffffffu, x[r], J);
+            if ((q > x[r]) == lower) x[r] = q;
         }
     }
 }
-
-// stages (k, j0), (k, j0/2), .., (k, 1), all inside the warp's chunk
-template <int R, typename Items>
-__device__ __forceinline__ void bitonic_local(typename Items::Item (&x)[R], int base, int lane, int k, int j0) {
-    for (int jj = j0; jj > 0; jj >>= 1) {
-        if (jj >= 32) {
-            const int d = jj >> 5;
-            if (d == 4) bitonic_thread_stage<R, 4, Items>(x, base, lane, k);
-            else if (d == 2) bitonic_thread_stage<R, 2, Items>(x, base, lane, k);
-            else bitonic_thread_stage<R, 1, Items>(x, base, lane, k);
-        } else {
-            const bool lower = (lane & jj) == 0;
+// the stages of k with j < 32 R
+template <int R> __device__ __forceinline__ void sort64_local(unsigned long long (&x)[R], int base, int lane, int k) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const bool up = ((base + r * 32 + lane) & k) == 0;
-                const typename Items::Item q = Items::shfl(x[r], jj);
-                const bool sw = lower ? (Items::before(q, x[r]) == up) : (Items::before(x[r], q) == up);
-                if (sw) x[r] = q;
-            }
-        }
-    }
+    for (int r = 0; r < R; ++r)
+        if ((base + 32 * r + lane) & k) x[r] = ~x[r];
+    if constexpr (R > 4) { if (k > 128) sort64_stage<R, 128>(x, lane); }
+    if constexpr (R > 2) { if (k > 64) sort64_stage<R, 64>(x, lane); }
+    if constexpr (R > 1) { if (k > 32) sort64_stage<R, 32>(x, lane); }
+    if (k > 16) sort64_stage<R, 16>(x, lane);
+    if (k > 8) sort64_stage<R, 8>(x, lane);
+    if (k > 4) sort64_stage<R, 4>(x, lane);
+    if (k > 2) sort64_stage<R, 2>(x, lane);
+    sort64_stage<R, 1>(x, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if ((base + 32 * r + lane) & k) x[r] = ~x[r];
 }
-
-template <int R, typename Items>
-__device__ void bitonic_sort_chunks(const Items& it, int n_pad) {
-    const int lane = threadIdx.x & 31;
-    const int CH = 32 * R, base = (threadIdx.x >> 5) * CH;
-    typename Items::Item x[R];
+template <int R> __device__ __forceinline__ void sort64_chunks(unsigned long long* key, int n_pad) {
+    constexpr int CH = 32 * R;
+    const int lane = threadIdx.x & 31, base0 = (threadIdx.x >> 5) * CH, step = (blockDim.x >> 5) * CH;
+    unsigned long long x[R];
+    for (int base = base0; base < n_pad; base += step) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) x[r] = it.load(base + r * 32 + lane);
-    for (int k = 2; k <= CH; k <<= 1) bitonic_local<R, Items>(x, base, lane, k, k >> 1);
+        for (int r = 0; r < R; ++r) x[r] = key[base + 32 * r + lane];
+#pragma unroll 1
+        for (int k = 2; k <= CH; k <<= 1) sort64_local<R>(x, base, lane, k);
 #pragma unroll
-    for (int r = 0; r < R; ++r) it.store(base + r * 32 + lane, x[r]);
+        for (int r = 0; r < R; ++r) key[base + 32 * r + lane] = x[r];
+    }
+#pragma unroll 1
     for (int k = 2 * CH; k <= n_pad; k <<= 1) {
+#pragma unroll 1
         for (int jj = k >> 1; jj >= CH; jj >>= 1) {
             __syncthreads();
-            bitonic_smem_stage(it, n_pad, k, jj);
+            for (int t = threadIdx.x; t < n_pad / 2; t += blockDim.x) {
+                const int i = ((t & ~(jj - 1)) << 1) | (t & (jj - 1));
+                const unsigned long long lo = key[i], hi = key[i + jj];
+                if ((hi > lo) == ((i & k) == 0)) {
+                    key[i] = hi;
+                    key[i + jj] = lo;
+                }
+            }
         }
         __syncthreads();
+        for (int base = base0; base < n_pad; base += step) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) x[r] = it.load(base + r * 32 + lane);
-        bitonic_local<R, Items>(x, base, lane, k, CH >> 1);
+            for (int r = 0; r < R; ++r) x[r] = key[base + 32 * r + lane];
+            sort64_local<R>(x, base, lane, k);
 #pragma unroll
-        for (int r = 0; r < R; ++r) it.store(base + r * 32 + lane, x[r]);
+            for (int r = 0; r < R; ++r) key[base + 32 * r + lane] = x[r];
+        }
     }
 }
-
-template <typename Items>
-__device__ void block_bitonic_sort(const Items& it, int n_pad) {
-    __syncthreads();
-    const int nw = blockDim.x >> 5;
-    const int ch = n_pad / nw;
-    if (ch * nw == n_pad && ch >= 32 && ch <= 256) {
-        if (ch == 32) bitonic_sort_chunks<1>(it, n_pad);
-        else if (ch == 64) bitonic_sort_chunks<2>(it, n_pad);
-        else if (ch == 128) bitonic_sort_chunks<4>(it, n_pad);
-        else bitonic_sort_chunks<8>(it, n_pad);
-    } else {
-        for (int k = 2; k <= n_pad; k <<= 1)
-            for (int jj = k >> 1; jj > 0; jj >>= 1) {
-                bitonic_smem_stage(it, n_pad, k, jj);
-                __syncthreads();
-            }
-    }
-    __syncthreads();
+// keys are padded to a power of two, one warp's chunk at least
+__host__ __device__ inline int sort64_pad(int n) {
+    int p = 32;
+    while (p < n) p <<= 1;
+    return p;
 }
-
-// In-place sort of (w, key, r) by merge_before over n_pad (power of 2) slots.
-template <typename T>
-__device__ void sort_survivors(T* s_w, uint32_t* s_key, int* s_r, int n_pad) {
-    block_bitonic_sort(SurvItems<T>{s_w, s_key, s_r}, n_pad);
+// place of a key among the n sorted ones
+__device__ __forceinline__ int sort64_find(const unsigned long long* key, int n, unsigned long long k) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (key[mid] > k) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+__device__ void block_sort64(unsigned long long* key, int n_pad) {
+    __syncthreads();
+    const int ch = n_pad / (blockDim.x >> 5);
+    if (ch <= 32) sort64_chunks<1>(key, n_pad);
+    else if (ch == 64) sort64_chunks<2>(key, n_pad);
+    else if (ch == 128) sort64_chunks<4>(key, n_pad);
+    else sort64_chunks<8>(key, n_pad);
+    __syncthreads();
 }
 
 // Block-wide exclusive scan of int flags; returns the total.  Starts with a barrier:
@@ -1267,20 +1254,29 @@ __device__ __forceinline__ void uf_unite(int* uf, int a, int b) {
 }
 
 // Shared-memory working set of the merge (per CTA); sizes are derived from the
-// survivor capacity S and map capacity G by merge_smem_bytes().
+// survivor capacity S and map capacity G by merge_shared_bytes() (filters) and
+// merge_list_bytes() (callers' lists).
 template <typename T> struct MergeScratch {
-    float* pf;            // S x 6: mean[0..3), cov diagonal [0..3) (prefilter data)
+    int S;                // capacity
+    float* pf;            // 3 x S: cov diagonal [0..3); behind it, where the view holds no FP32
+                          // means, 3 x S: mean[0..3) (prefilter data)
     uint8_t* flag;        // S: merged
     uint8_t* is_center;   // S
     int* lab;             // S: union-find parent, then the component's root
     int* cidx;            // S: component index of a root; later the queue of large components
     int* start;           // S + 1: member range of each component in perm
-    int* fill;            // S
-    int* perm;            // cap: survivors grouped by component (first: survivors in u order)
+    int* fill;            // S: member ranks within a component, then scratch of the large components
+    int* perm;            // survivors grouped by component (first: survivors in u order)
     uint32_t* masks;      // (blockDim/32) x nchunk member masks
     int nchunk;
 };
 
+// Up to this many survivors are ordered by counting, for each, those before it, and paired by
+// scanning all pairs: steps of a few independent instructions without barriers, n of them per
+// survivor and n / 2, against two bitonic sorts of next_pow2(n) with 20 barriers each.  Merge of
+// 256 parents with 66 survivors 32 -> 26 us, 1024 with 150 99 -> 93 us; at 253 survivors the
+// sorts win (0.52 against 0.54 ms at 4096 parents).
+constexpr int kPairScan = 160;
 constexpr int kSmallComp = 8;       // components up to this size are merged by one thread
 constexpr int kMergeThreads = 256;   // threads of a parent's merge block (8 warps)
 template <typename T> constexpr int kMergeBlocks = sizeof(T) == 4 ? 3 : 2;   // blocks per SM by registers
@@ -1291,77 +1287,75 @@ __host__ __device__ inline int next_pow2(int x) {
     return p;
 }
 
-// sort capacity (survivors, then map entries), in elements
-__host__ __device__ inline int merge_sort_cap(int S, int G) {
-    int a = next_pow2(S), b = S + G;
-    return a > b ? a : b;
+// The limit that scphd_create and scphd_batch_create hold max_survivors (S) and max_gaussians
+// (G) to, in bytes of a merge block; what a block takes is less (merge_shared_bytes).
+template <typename T> inline size_t merge_limit_bytes(int S, int G, int nwarps) {
+    const size_t pad = next_pow2(S), sum = (size_t)S + G, cap = pad > sum ? pad : sum;
+    const size_t stage = ((6 * (size_t)S + 21) * sizeof(T) + 4 * (size_t)S + 15) & ~(size_t)15;
+    return stage + cap * (sizeof(T) + 12) + 4 * (6 * (size_t)S > sum ? 6 * (size_t)S : sum) + 16 * (size_t)S + 4 +
+           (size_t)nwarps * ((S + 31) / 32) * 4 + 2 * (size_t)S + 64;
 }
 
-// Survivor staging of the filter's merge (KalmanView) in front of the scratch: means
-// (S x 6), the birth covariance (21) and covariance-row indices (S).  A caller's rows
-// (ListView) are read in place and stage nothing.  (Staging the G posterior
-// covariances as well was measured slower: the copy costs more than the reads save.)
-template <typename T> __host__ __device__ inline size_t merge_stage_bytes(int S, bool stage) {
-    return stage ? (((6 * (size_t)S + 21) * sizeof(T) + 4 * (size_t)S + 15) & ~(size_t)15) : 0;
+// shared memory of a caller's list of up to S components (k_merge_list)
+template <typename T> inline size_t merge_list_bytes(int S, int nwarps) {
+    const size_t pad = sort64_pad(S);
+    return pad * (sizeof(T) + 8 + 4 + 4) + 4 * (9 * (size_t)S + S + 1) + (size_t)nwarps * ((S + 31) / 32) * 4 + 2 * (size_t)S;
 }
-template <typename T> inline size_t merge_smem_bytes(int S, int G, int nwarps, bool stage) {
-    const size_t cap = merge_sort_cap(S, G), nchunk = (S + 31) / 32;
-    const size_t pf = 6 * (size_t)S * sizeof(float), pos = (size_t)(S + G) * 4;   // pos aliases pf
-    return merge_stage_bytes<T>(S, stage) + cap * (sizeof(T) + 8) + (pf > pos ? pf : pos) + 3 * (size_t)S * 4 +
-           cap * 4 + (size_t)(S + 1) * 4 + (size_t)nwarps * nchunk * 4 + 2 * (size_t)S + 64;
-}
-// shared memory of a caller's list of up to S components (merge_smem_bytes(S, 0, ., false))
 template <typename T>
-__device__ inline void carve_merge_list(unsigned char* smem, int S, T*& s_w, uint32_t*& s_key,
-                                        int*& s_r, int*& s_pos, MergeScratch<T>& ms) {
-    const int cap = merge_sort_cap(S, 0);
+__device__ inline void carve_merge_list(unsigned char* smem, int S, T*& s_w, unsigned long long*& s_key, int*& s_r,
+                                        int*& s_pos, MergeScratch<T>& ms) {
+    const int pad = sort64_pad(S);
     s_w = reinterpret_cast<T*>(smem);
-    s_key = reinterpret_cast<uint32_t*>(s_w + cap);
-    s_r = reinterpret_cast<int*>(s_key + cap);
-    ms.pf = reinterpret_cast<float*>(s_r + cap);
+    s_key = reinterpret_cast<unsigned long long*>(s_w + pad);
+    s_r = reinterpret_cast<int*>(s_key + pad);
+    ms.S = S;
+    ms.pf = reinterpret_cast<float*>(s_r + pad);
     s_pos = reinterpret_cast<int*>(ms.pf);   // positions are used only once the prefilter rows are dead
     ms.lab = reinterpret_cast<int*>(ms.pf + 6 * S);
     ms.cidx = ms.lab + S;
     ms.fill = ms.cidx + S;
     ms.perm = ms.fill + S;
-    ms.start = ms.perm + cap;
+    ms.start = ms.perm + pad;
     ms.nchunk = (S + 31) / 32;
     ms.masks = reinterpret_cast<uint32_t*>(ms.start + S + 1);
     ms.flag = reinterpret_cast<uint8_t*>(ms.masks + (blockDim.x / 32) * ms.nchunk);
     ms.is_center = ms.flag + S;
 }
 
-// The filter's merge keeps less at a time than that: arrays that are never live together
-// share their bytes.  The means' area holds the sort keys before them and the new map's
-// weights after them, the ranks' holds the member lists, the u keys' the component indices,
-// the prefilter's the output positions.  (merge_smem_bytes stays the limit that scphd_create
-// and scphd_batch_create check.)
+// The filter's merge: arrays that are never live together share their bytes.  The means' area holds the sort keys before them and the new map's weights after
+// them; the u keys' holds the ranks before them, the component indices and member lists after
+// them; the prefilter's the output positions.  In FP32 the prefilter's u, v, d are the means'
+// (6 x S arrays), in FP64 copies.
 template <typename T> __host__ __device__ inline size_t merge_area_bytes(int S, int G) {
-    const size_t stage = merge_stage_bytes<T>(S, true), keys = sizeof(T) == 4 ? 8 * (size_t)next_pow2(S) : 0;
+    const size_t stage = 6 * (size_t)S * sizeof(T) + 4 * (size_t)S, keys = 8 * (size_t)sort64_pad(S);
     const size_t out = (size_t)(S + G) * sizeof(T);
     const size_t m = stage > keys ? (stage > out ? stage : out) : (keys > out ? keys : out);
     return (m + 15) & ~(size_t)15;
 }
+template <typename T> __host__ __device__ inline size_t merge_pf_words(int S, int G) {
+    const size_t pf = (sizeof(T) == 4 ? 3 : 6) * (size_t)S;
+    return pf > (size_t)(S + G) ? pf : (size_t)(S + G);
+}
 template <typename T> __host__ __device__ inline size_t merge_shared_bytes(int S, int G, int nwarps) {
-    const size_t pad = next_pow2(S), pf = 6 * (size_t)S > (size_t)(S + G) ? 6 * (size_t)S : (size_t)(S + G);
-    return merge_area_bytes<T>(S, G) + pad * (sizeof(T) + 8) + 4 * (pf + 3 * (size_t)S + 1) +
-           (size_t)nwarps * ((S + 31) / 32) * 4 + 2 * (size_t)S;
+    return merge_area_bytes<T>(S, G) + (size_t)((S + 3) & ~3) * sizeof(T) + 8 * (size_t)sort64_pad(S) +
+           4 * (merge_pf_words<T>(S, G) + 3 * (size_t)S + 1) + (size_t)nwarps * ((S + 31) / 32) * 4 + 2 * (size_t)S;
 }
 template <typename T>
-__device__ inline void carve_merge_shared(unsigned char* smem, int S, int G, T*& s_w, uint32_t*& s_key, int*& s_r,
+__device__ inline void carve_merge_shared(unsigned char* smem, int S, int G, T*& s_w, unsigned long long*& s_key, int*& s_r,
                                           int*& s_pos, T*& s_out, MergeScratch<T>& ms) {
-    const int pad = next_pow2(S);
+    const int pad = sort64_pad(S);
     s_out = reinterpret_cast<T*>(smem);
     s_w = reinterpret_cast<T*>(smem + merge_area_bytes<T>(S, G));
-    s_key = reinterpret_cast<uint32_t*>(s_w + pad);
-    s_r = reinterpret_cast<int*>(s_key + pad);
-    ms.pf = reinterpret_cast<float*>(s_r + pad);
+    s_key = reinterpret_cast<unsigned long long*>(s_w + ((S + 3) & ~3));
+    s_r = reinterpret_cast<int*>(s_key);
+    ms.S = S;
+    ms.pf = reinterpret_cast<float*>(s_key + pad);
     s_pos = reinterpret_cast<int*>(ms.pf);
-    ms.lab = reinterpret_cast<int*>(ms.pf + (6 * S > S + G ? 6 * S : S + G));
+    ms.lab = reinterpret_cast<int*>(ms.pf + merge_pf_words<T>(S, G));
     ms.fill = ms.lab + S;
     ms.start = ms.fill + S;
     ms.cidx = reinterpret_cast<int*>(s_key);
-    ms.perm = s_r;
+    ms.perm = ms.cidx + pad;
     ms.nchunk = (S + 31) / 32;
     ms.masks = reinterpret_cast<uint32_t*>(ms.start + S + 1);
     ms.flag = reinterpret_cast<uint8_t*>(ms.masks + (blockDim.x / 32) * ms.nchunk);
@@ -1375,8 +1369,8 @@ __device__ inline void carve_merge_shared(unsigned char* smem, int S, int G, T*&
 // capacity leaves an SM half the blocks that registers allow (`blocks`) or fewer, parents are
 // merged by a launch sized for `blocks`, and the few with more survivors, which it lists, by
 // a second one at the full capacity (4 us when the list is empty): 4.6 -> 2.8 ms and, in
-// FP64, 1.96 -> 1.32 ms at those sizes.  From two blocks to three there is nothing to gain
-// (FP32 at 968 survivors: 0.62 ms either way).
+// FP64, 1.96 -> 1.32 ms at those sizes.  From two blocks to three the gain is 5 %, less at
+// few parents: that is left to the layout (FP32 at 968 survivors: three fit).
 template <typename T> inline int merge_launch_cap(int Scap, int G, int threads, int blocks) {
     auto room = [](int n) { return (size_t)228 * 1024 / n - 1024 - 3584; };   // less what a block reserves, and static
     if (merge_shared_bytes<T>(Scap, G, threads / 32) <= room(blocks / 2 + 1)) return Scap;
@@ -1385,12 +1379,15 @@ template <typename T> inline int merge_launch_cap(int Scap, int G, int threads, 
     return S >= G ? S : Scap;   // a parent seldom has fewer survivors than its map may hold
 }
 
-__device__ __forceinline__ bool could_merge_f(const float* a, const float* b, float min_sep, float margin) {
+// the prefilter's values of component i: pm[k S + i] the mean's u, v, d, pf[k S + i] the
+// covariance's diagonal entries (arrays, so that lanes of consecutive i read consecutive words)
+__device__ __forceinline__ bool could_merge_f(const float* pm, const float* pf, int S, int i, int j, float min_sep,
+                                              float margin) {
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        float d = a[k] - b[k];
-        ok = ok && (d * d <= min_sep * (a[3 + k] + b[3 + k]) * margin);
+        const float d = pm[k * S + i] - pm[k * S + j];
+        ok = ok && (d * d <= min_sep * (pf[k * S + i] + pf[k * S + j]) * margin);
     }
     return ok;
 }
@@ -1432,7 +1429,8 @@ __device__ void merge_members_thread(const View& v, const T* s_w, const int* mem
         } else {
             v.mean(i, mu);
         }
-        const T* sc = v.cov(i);
+        T sc[21];
+        v.cov(i, sc);
 #pragma unroll
         for (int a = 0; a < 6; ++a) d[a] = row[1 + a] - mu[a];
 #pragma unroll
@@ -1513,11 +1511,6 @@ __device__ uint64_t select_kth_largest(const T* w, int n, int k) {
     return prefix;
 }
 
-// In-place bitonic sort of (key, payload) ascending by key over n_pad (power of 2) slots.
-__device__ void sort_keys(uint32_t* key, int* val, int n_pad) {
-    block_bitonic_sort(KeyItems{key, val}, n_pad);
-}
-
 // Greedy reduction of phdUpdateMergeKernel (src/kernels.cu:693-866) over n
 // survivors already sorted into the reference's argmax order: the next centre is
 // the first unmerged survivor, every unmerged survivor within squared Mahalanobis
@@ -1532,102 +1525,113 @@ __device__ void sort_keys(uint32_t* key, int* val, int n_pad) {
 // or n.  Block-wide call.
 template <typename T, typename View>
 __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int n, MergeScratch<T> ms,
-                                uint32_t* ukey, T min_sep, T* sparse, int* member_out,
+                                unsigned long long* ukey, T min_sep, T* sparse, int* member_out,
                                 unsigned long long* counters) {
     __shared__ int s_ncomp, s_take, s_nlarge, s_take_large, s_stop, s_evals;
     __shared__ int s_tmp[40];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float fsep = (float)min_sep, fmargin = 1.01f;
+    const float* pm = v.float_means(ms.pf + 3 * ms.S);
     for (int i = tid; i < n; i += blockDim.x) {
         T mu[6];
         v.mean(i, mu);
         const T* cv = v.cov(i);
-        float* pf = ms.pf + i * 6;
-        pf[0] = (float)mu[0]; pf[1] = (float)mu[1]; pf[2] = (float)mu[2];
-        pf[3] = (float)cv[0]; pf[4] = (float)cv[2]; pf[5] = (float)cv[5];
+        ms.pf[i] = (float)cv[0]; ms.pf[ms.S + i] = (float)cv[2]; ms.pf[2 * ms.S + i] = (float)cv[5];
+        if (!View::kFloatMeans)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) ms.pf[(3 + k) * ms.S + i] = (float)mu[k];
         ms.flag[i] = 0;
         ms.is_center[i] = 0;
         ms.lab[i] = i;
     }
     if (tid == 0) { s_ncomp = 0; s_take = 0; s_nlarge = 0; s_take_large = 0; s_stop = n; s_evals = 0; }
-    __syncthreads();
-    // "may merge" edges -> union-find.  |du| <= sqrt(sep*margin*(Suu_i + max Suu)) is
-    // necessary for the bound on u, so with the survivors in u order each one scans
-    // forward only over that window.
-    __shared__ float s_maxsuu;
-    {
-        float mx = 0.f;
+    // "may merge" edges -> union-find
+    if (View::kScansPairs && n <= kPairScan) {
+        // every pair once, without a barrier or a sort: thread i scans the n / 2 components
+        // after it, round the end, so that all scan alike.  The bound on u alone (a little
+        // wider than could_merge_f's) drops nearly all; u and the widened variances are held
+        // twice in a row so that the scan needs no wrapping.
+        float* pu = reinterpret_cast<float*>(ukey);
+        float* ps = reinterpret_cast<float*>(ms.fill);   // 2 n <= 2 S: fill and start
+        __syncthreads();   // (the ranks are staged; the prefilter's values are written)
         for (int i = tid; i < n; i += blockDim.x) {
-            mx = fmaxf(mx, ms.pf[i * 6 + 3]);
-            const float u = ms.pf[i * 6 + 0];
-            uint32_t bits = __float_as_uint(u);
-            ukey[i] = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);   // orderable float key
-            ms.perm[i] = i;
+            const float u = pm[i], w = ms.pf[i] * (fsep * fmargin * 1.0001f);
+            pu[i] = pu[n + i] = u;
+            ps[i] = ps[n + i] = w;
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += blockDim.x) {
+            const float u = pu[i], w = ps[i];
+            const int last = n - 1 - (n & 1 ? 0 : (i >= n / 2));   // n even: the opposite pair once
+            const int half = last / 2 + (n & 1 ? 0 : last & 1);
+            // hits of up to 32 components collected without a branch (some lane of the warp
+            // has one in most groups), then looked at one by one
+            for (int k0 = 1; k0 <= half; k0 += 32) {
+                const int kn = min(32, half - k0 + 1);
+                uint32_t hits = 0;
+#pragma unroll 8
+                for (int q = 0; q < kn; ++q) {
+                    const float du = u - pu[i + k0 + q];
+                    if (du * du <= w + ps[i + k0 + q]) hits |= 1u << q;
+                }
+                for (; hits; hits &= hits - 1) {
+                    const int x = i + k0 + __ffs(hits) - 1, j = x < n ? x : x - n;
+                    if (could_merge_f(pm, ms.pf, ms.S, i, j, fsep, fmargin)) uf_unite(ms.lab, i, j);
+                }
+            }
+        }
+    } else {
+        // |du| <= sqrt(sep*margin*(Suu_i + max Suu)) is necessary for the bound on u, so with
+        // the survivors in u order each one scans forward only over that window.
+        __shared__ float s_maxsuu;
+        __syncthreads();
+        float mx = 0.f;
+        const int np2 = sort64_pad(n);
+        for (int i = tid; i < np2; i += blockDim.x) {
+            unsigned long long key = 0ull;
+            if (i < n) {   // ascending u: complemented
+                mx = fmaxf(mx, ms.pf[i]);
+                key = ~((unsigned long long)float_order(pm[i]) << 32 | (uint32_t)i);
+            }
+            ukey[i] = key;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (tid == 0) s_maxsuu = 0.f;
         __syncthreads();
         if (lane == 0) atomicMax(reinterpret_cast<int*>(&s_maxsuu), __float_as_int(mx));   // mx >= 0
-        const int np2 = next_pow2(n);
-        for (int i = n + tid; i < np2; i += blockDim.x) { ukey[i] = 0xffffffffu; ms.perm[i] = 0x7fffffff; }
-        __syncthreads();
-        sort_keys(ukey, ms.perm, np2);
-    }
-    const float maxsuu = s_maxsuu;
-    for (int q = tid; q < n; q += blockDim.x) {
-        const int i = ms.perm[q];
-        float a[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) a[k] = ms.pf[i * 6 + k];
-        const float reach = sqrtf(fsep * fmargin * (a[3] + maxsuu)) * 1.0001f;
-        for (int q2 = q + 1; q2 < n; ++q2) {
-            const int j = ms.perm[q2];
-            const float* bj = ms.pf + j * 6;
-            if (bj[0] - a[0] > reach) break;
-            if (could_merge_f(a, bj, fsep, fmargin)) uf_unite(ms.lab, i, j);
+        block_sort64(ukey, np2);
+        const float maxsuu = s_maxsuu;
+        for (int q = tid; q < n; q += blockDim.x) {
+            const int i = (int)~(uint32_t)ukey[q];
+            const float u = pm[i];
+            const float reach = sqrtf(fsep * fmargin * (ms.pf[i] + maxsuu)) * 1.0001f;
+            for (int q2 = q + 1; q2 < n; ++q2) {
+                const int j = (int)~(uint32_t)ukey[q2];
+                if (pm[j] - u > reach) break;
+                if (could_merge_f(pm, ms.pf, ms.S, i, j, fsep, fmargin)) uf_unite(ms.lab, i, j);
+            }
         }
     }
     __syncthreads();
+    // components: numbered, their members counted (each keeps its place), and listed; a
+    // component's members are put into ascending order by whoever merges it
     for (int i = tid; i < n; i += blockDim.x) {
         if (uf_find(ms.lab, i) == i) {
             int c = atomicAdd(&s_ncomp, 1);
             ms.cidx[i] = c;
             ms.start[c] = 0;
-            ms.fill[c] = 0;
         }
     }
-    __syncthreads();
-    for (int i = tid; i < n; i += blockDim.x) ms.lab[i] = uf_find(ms.lab, i);
     __syncthreads();
     const int ncomp = s_ncomp;
-    for (int i = tid; i < n; i += blockDim.x) atomicAdd(&ms.start[ms.cidx[ms.lab[i]]], 1);
-    __syncthreads();
+    for (int i = tid; i < n; i += blockDim.x) {
+        const int c = ms.cidx[uf_find(ms.lab, i)];
+        ms.fill[i] = atomicAdd(&ms.start[c], 1);
+    }
     block_exclusive_scan(ms.start, ncomp, s_tmp);
     if (tid == 0) ms.start[ncomp] = n;
-    __syncthreads();
-    // members of each component in ascending order (chunks in order, ranks by lane)
-    if (warp == 0) {
-        for (int base = 0; base < n; base += 32) {
-            const int i = base + lane;
-            const bool valid = i < n;
-            const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-            if (valid) {
-                const int c = ms.cidx[ms.lab[i]];
-                const unsigned grp = __match_any_sync(vmask, c);
-                const int leader = __ffs(grp) - 1;
-                const int rank = __popc(grp & ((1u << lane) - 1u));
-                int off = 0;
-                if (lane == leader) {
-                    off = ms.fill[c];
-                    ms.fill[c] = off + __popc(grp);
-                }
-                off = __shfl_sync(grp, off, leader);
-                ms.perm[ms.start[c] + off + rank] = i;
-            }
-            __syncwarp();
-        }
-    }
+    for (int i = tid; i < n; i += blockDim.x) ms.perm[ms.start[ms.cidx[uf_find(ms.lab, i)]] + ms.fill[i]] = i;
     __syncthreads();
     int evals = 0;
     // small components: one thread each; large ones are queued for the warps
@@ -1639,7 +1643,13 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
             ms.cidx[atomicAdd(&s_nlarge, 1)] = c;   // roots' indices are no longer needed
             continue;
         }
-        const int* mem = ms.perm + s0;
+        int* mem = ms.perm + s0;
+        for (int k = 1; k < cnt; ++k) {   // ascending
+            const int x = mem[k];
+            int q = k;
+            for (; q > 0 && mem[q - 1] > x; --q) mem[q] = mem[q - 1];
+            mem[q] = x;
+        }
         uint32_t done = 0;
         while (true) {
             const int k0 = __ffs(~done) - 1;
@@ -1647,9 +1657,7 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
             const int cc = mem[k0];
             T cmu[6], ccov[21];
             v.mean(cc, cmu);
-            const T* cp = v.cov(cc);
-#pragma unroll
-            for (int q = 0; q < 21; ++q) ccov[q] = cp[q];
+            v.cov(cc, ccov);
             uint32_t mbits = 0;
             for (int k = k0; k < cnt; ++k) {
                 if ((done >> k) & 1u) continue;
@@ -1658,11 +1666,12 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
                     mbits |= 1u << k;
                     continue;
                 }
-                if (!could_merge_f(ms.pf + cc * 6, ms.pf + i * 6, fsep, fmargin)) continue;
+                if (!could_merge_f(pm, ms.pf, ms.S, cc, i, fsep, fmargin)) continue;
                 ++evals;
-                T mu[6];
+                T mu[6], cv[21];
                 v.mean(i, mu);
-                if (mahal6(cmu, ccov, mu, v.cov(i)) < min_sep) mbits |= 1u << k;
+                v.cov(i, cv);
+                if (mahal6(cmu, ccov, mu, cv) < min_sep) mbits |= 1u << k;
             }
             if (!mbits) {   // merged weight 0: the reference's loop ends (kernels.cu:783-784)
                 atomicMin(&s_stop, cc);
@@ -1685,8 +1694,17 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
         if (q >= s_nlarge) break;
         const int c = ms.cidx[q];
         const int s0 = ms.start[c], cnt = ms.start[c + 1] - s0;
-        const int* mem = ms.perm + s0;
+        int* mem = ms.perm + s0;
         const int nch = (cnt + 31) >> 5;
+        for (int k = lane; k < cnt; k += 32) {   // ascending: each member to its rank, by way of fill
+            const int x = mem[k];
+            int rank = 0;
+            for (int q2 = 0; q2 < cnt; ++q2) rank += mem[q2] < x;
+            ms.fill[s0 + rank] = x;
+        }
+        __syncwarp();
+        for (int k = lane; k < cnt; k += 32) mem[k] = ms.fill[s0 + k];
+        __syncwarp();
         int next = 0;
         while (true) {
             int k0 = -1;
@@ -1701,20 +1719,19 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
             const int cc = mem[k0];
             T cmu[6], ccov[21];
             v.mean(cc, cmu);
-            const T* cp = v.cov(cc);
-#pragma unroll
-            for (int qq = 0; qq < 21; ++qq) ccov[qq] = cp[qq];
+            v.cov(cc, ccov);
             bool any = false;
             for (int ch = k0 >> 5; ch < nch; ++ch) {
                 const int k = ch * 32 + lane;
                 bool m = false;
                 if (k >= k0 && k < cnt) {
                     const int i = mem[k];
-                    if (!ms.flag[i] && could_merge_f(ms.pf + cc * 6, ms.pf + i * 6, fsep, fmargin)) {
+                    if (!ms.flag[i] && could_merge_f(pm, ms.pf, ms.S, cc, i, fsep, fmargin)) {
                         ++evals;
-                        T mu[6];
+                        T mu[6], cv[21];
                         v.mean(i, mu);
-                        m = mahal6(cmu, ccov, mu, v.cov(i)) < min_sep;
+                        v.cov(i, cv);
+                        m = mahal6(cmu, ccov, mu, cv) < min_sep;
                     }
                 }
                 const unsigned bal = __ballot_sync(0xffffffffu, m);
@@ -1807,33 +1824,22 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
         if (tid == 0) b.src_tmp[atomicAdd(b.flags + 3, 1)] = p;
         return;
     }
-    const int n_pad = next_pow2(n);
     T* s_w;
-    uint32_t* s_key;
+    unsigned long long* s_key;
     int* s_r;
     int* s_pos;
     T* s_out;
     MergeScratch<T> ms;
     carve_merge_shared<T>(smem, S, prm.Gcap, s_w, s_key, s_r, s_pos, s_out, ms);
     __shared__ int s_tmp[40];
-    // FP32: packed sort keys in the survivor staging area (free until the survivors are
-    // staged; 8 n_pad <= 16 Scap bytes fit in its 28 Scap); FP64: (weight, tie key, rank)
+    // sort keys in the survivor staging area (free until the survivors are staged): the order
+    // key's bits above the complement of the tie key
     unsigned long long* s_pk = reinterpret_cast<unsigned long long*>(smem);
-    for (int i = tid; i < n_pad; i += blockDim.x) {
-        if (sizeof(T) == 4) {
-            s_pk[i] = i < n ? pack_survivor((float)b.surv_w[(size_t)p * prm.Scap + i],
-                                            (uint32_t)b.surv_r[(size_t)p * prm.Scap + i])
-                            : 0ull;
-        } else if (i < n) {
-            s_w[i] = b.surv_w[(size_t)p * prm.Scap + i];
-            s_r[i] = b.surv_r[(size_t)p * prm.Scap + i];
-            s_key[i] = tie_key((uint32_t)s_r[i]);
-        } else {
-            s_w[i] = T(-1);
-            s_key[i] = 0xffffffffu;
-            s_r[i] = 0x7fffffff;
-        }
-    }
+    const T* surv_w = b.surv_w + (size_t)p * prm.Scap;
+    const int* surv_r = b.surv_r + (size_t)p * prm.Scap;
+    const bool counted = n <= kPairScan;
+    const int n_pad = counted ? (n + 1) & ~1 : sort64_pad(n);
+    for (int i = tid; i < n_pad; i += blockDim.x) s_pk[i] = i < n ? pack_survivor(order_key(surv_w[i]), (uint32_t)surv_r[i]) : 0ull;
     // parent log-likelihood: sum_m ell + sum_j w_j (.cu:1813-1849), FP64, in an order
     // that does not depend on the block's width (128 or 256 threads, stage kernel or
     // fused): 256 lane partials, a butterfly within each group of 32, the 8 group
@@ -1842,7 +1848,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     for (int v = tid; v < 256; v += blockDim.x) {
         double part = 0;
         for (int mm = v; mm < M; mm += 256) part += (double)b.ell[(size_t)p * prm.Mcap + mm];
-        for (int j = v; j < G; j += 256) part += (double)b.fit[((size_t)p * prm.Gcap + j) * kRow];
+        for (int j = v; j < G; j += 256) part += (double)b.wts[((size_t)p * prm.Gcap + j) * 2];
         s_part[v] = part;
     }
     __syncthreads();
@@ -1856,17 +1862,30 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
         }
         if (tid == 0) b.loglik[p] = t;
     }
-    if (sizeof(T) == 4) {
-        block_bitonic_sort(PackedSurvItems{s_pk}, n_pad);
-        for (int i = tid; i < n_pad; i += blockDim.x) {
-            const unsigned long long v = s_pk[i];
-            s_w[i] = i < n ? (T)__uint_as_float((uint32_t)(v >> 32)) : T(-1);
-            s_r[i] = i < n ? (int)untie_key(~(uint32_t)v) : 0x7fffffff;
+    if (counted) {
+        // a survivor's place is the number of larger keys (they are distinct)
+        for (int i = tid; i < n; i += blockDim.x) {
+            const unsigned long long key = s_pk[i];
+            int at = 0;
+#pragma unroll 4
+            for (int j = 0; j < n; j += 2) {
+                const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(s_pk + j);
+                at += o.x > key;
+                at += o.y > key;
+            }
+            s_w[at] = surv_w[i];
+            s_r[at] = surv_r[i];
         }
-        __syncthreads();   // the staging below reuses the key area
     } else {
-        sort_survivors(s_w, s_key, s_r, n_pad);
+        block_sort64(s_pk, n_pad);
+        for (int i = tid; i < n; i += blockDim.x) {
+            const T w = surv_w[i];
+            const int r = surv_r[i], at = sort64_find(s_pk, n, pack_survivor(order_key(w), (uint32_t)r));
+            s_w[at] = w;
+            s_r[at] = r;
+        }
     }
+    __syncthreads();   // the staging below reuses the key area
     KalmanSource<T, K> src;
     src.fit = b.fit + (size_t)p * prm.Gcap * kRow;
     src.prep = b.prep + (size_t)p * prm.Gcap * kPrep;
@@ -1875,32 +1894,24 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     src.M = M;
     src.bmean[0] = 0; src.bmean[1] = 0;
     src.bmean[2] = (T)prm.d0; src.bmean[3] = (T)prm.vu0; src.bmean[4] = (T)prm.vv0; src.bmean[5] = (T)prm.vd0;
-    for (int i = 0; i < 21; ++i) src.bcov[i] = 0;
-    src.bcov[tri(0, 0)] = (T)prm.model.var[0];
-    src.bcov[tri(1, 1)] = (T)prm.model.var[1];
-    src.bcov[tri(2, 2)] = (K == 3) ? (T)prm.model.var[2] : (T)prm.var_d0;
-    src.bcov[tri(3, 3)] = (T)prm.var_vu0;
-    src.bcov[tri(4, 4)] = (T)prm.var_vv0;
-    src.bcov[tri(5, 5)] = (T)prm.var_vd0;
     // survivors' means and covariance rows staged once (each is read several times)
     KalmanView<T> view;
     {
         T* st_mu = reinterpret_cast<T*>(smem);
-        T* st_bcov = st_mu + 6 * S;
-        int* st_cj = reinterpret_cast<int*>(st_bcov + 21);
+        int* st_cj = reinterpret_cast<int*>(st_mu + 6 * S);
         for (int i = tid; i < n; i += blockDim.x) {
             const int r = s_r[i];
             T mu[6];
             src.mean(r, mu);
 #pragma unroll
-            for (int a = 0; a < 6; ++a) st_mu[i * 6 + a] = mu[a];
+            for (int a = 0; a < 6; ++a) st_mu[a * S + i] = mu[a];
             st_cj[i] = r < G * M ? r % G : -1;
         }
-        if (tid < 21) st_bcov[tid] = src.bcov[tid];
         view.covs = src.prep + kPrepCov;
         view.mu = st_mu;
+        view.S = S;
         view.cj = st_cj;
-        view.bcov = st_bcov;
+        view.bcov = b.birth + kPrepCov;
         __syncthreads();
     }
     T* sparse = b.mtmp + (size_t)p * prm.Scap * kRow;
@@ -1918,7 +1929,6 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     for (int e = tid; e < n_out; e += blockDim.x) b.mlist[(size_t)p * prm.Scap + e] = centre_of[e];
     // new map: merged components then retained non-detection clouds (.cu:1923-2058);
     // entries e < n_out are merged, e >= n_out are the Gaussians j = e - n_out
-    const T minw = (T)prm.min_weight;
     const int n_all = n_out + G;
     int n_valid_part = 0;
     for (int e = tid; e < n_all; e += blockDim.x) {
@@ -1926,9 +1936,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
         if (e < n_out) {
             w = sparse[(size_t)centre_of[e] * kRow];
         } else {
-            const T* fr = b.fit + ((size_t)p * prm.Gcap + (e - n_out)) * kRow;
-            const T wnd = nd_weight(fr[0], fr[1]);
-            w = (wnd >= minw) ? wnd : T(-1);   // -1: not retained
+            w = b.wts[((size_t)p * prm.Gcap + (e - n_out)) * 2 + 1];   // -1: not retained
         }
         s_out[e] = w;
         n_valid_part += w >= T(0);
@@ -2446,7 +2454,7 @@ __global__ void __launch_bounds__(256) k_materialize(Params prm, Bufs<T> b, int 
 
 // ---------------------------------------------------------------- stand-alone merge
 // phdUpdateMergeKernel on an explicit component list (rows of kRow) with prune flags;
-// shared memory as merge_smem_bytes<T>(n_all + 1, 0, 4, false).
+// shared memory as merge_list_bytes<T>(n_all + 1, 4).
 template <typename T>
 __global__ void __launch_bounds__(128) k_merge_list(const T* rows, const uint8_t* flags_in, int n_all,
                                                     T min_sep, T* sparse, T* out, int* n_out_p, int* member_of) {
@@ -2458,10 +2466,9 @@ __global__ void __launch_bounds__(128) k_merge_list(const T* rows, const uint8_t
         s_n = n;
     }
     __syncthreads();
-    const int n = s_n;
-    const int n_pad = next_pow2(n);
+    const int n = s_n, n_pad = sort64_pad(n);
     T* s_w;
-    uint32_t* s_key;
+    unsigned long long* s_key;
     int* s_r;
     int* s_pos;
     MergeScratch<T> ms;
@@ -2469,16 +2476,18 @@ __global__ void __launch_bounds__(128) k_merge_list(const T* rows, const uint8_t
     if (threadIdx.x == 0) {
         int k = 0;
         for (int i = 0; i < n_all; ++i)
-            if (!flags_in[i]) {
-                s_w[k] = rows[(size_t)i * kRow];
-                s_r[k] = i;
-                s_key[k] = tie_key((uint32_t)i);
-                ++k;
-            }
-        for (; k < n_pad; ++k) { s_w[k] = T(-1); s_key[k] = 0xffffffffu; s_r[k] = 0x7fffffff; }
+            if (!flags_in[i]) s_key[k++] = pack_survivor(order_key(rows[(size_t)i * kRow]), (uint32_t)i);
+        for (; k < n_pad; ++k) s_key[k] = 0ull;
     }
+    block_sort64(s_key, n_pad);
+    for (int i = threadIdx.x; i < n_all; i += blockDim.x)
+        if (!flags_in[i]) {
+            const T w = rows[(size_t)i * kRow];
+            const int at = sort64_find(s_key, n, pack_survivor(order_key(w), (uint32_t)i));
+            s_w[at] = w;
+            s_r[at] = i;
+        }
     __syncthreads();
-    sort_survivors(s_w, s_key, s_r, n_pad);
     ListView<T> view{rows, s_r};
     const int stop = merge_components<T>(view, s_w, s_r, n, ms, s_key, min_sep, sparse, member_of, nullptr);
     for (int i = threadIdx.x; i < n; i += blockDim.x) s_pos[i] = (i < stop && ms.is_center[i]) ? 1 : 0;
