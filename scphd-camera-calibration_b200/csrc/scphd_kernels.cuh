@@ -888,8 +888,18 @@ __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>
                 const T c = t[0];
                 if (!(c > tneg_inf<T>())) continue;
                 const T lt = pair_term(t);
-                if (lt > mx) { acc = acc * exp_w(mx - lt) + T(1); mx = lt; }   // online log-sum-exp
-                else acc += exp_w(lt - mx);
+                // FP64 exponentials that cannot change the sum are not taken (most pairs are far
+                // apart; 0.73 -> 0.40 ms at 4096 parents x 256 Gaussians): the sum holds its
+                // largest term as 1, so a term below e^-38 < 2^-54 is rounded off, and so is what
+                // a new largest term more than 60 above scales down (at most G 2^-86)
+                if (lt > mx) {   // online log-sum-exp
+                    const T d = mx - lt;
+                    acc = !kB2 && d < T(-60) ? T(1) : acc * exp_w(d) + T(1);
+                    mx = lt;
+                } else {
+                    const T d = lt - mx;
+                    if (kB2 || !(d <= T(-38))) acc += exp_w(d);
+                }
                 if (lt >= cand_min) {
                     if (n_cand < kLikCand) s_cand[n_cand * blockDim.x + threadIdx.x] = k;
                     ++n_cand;
