@@ -364,9 +364,8 @@ __device__ __forceinline__ void cloud_fit_f32_body(const Params& prm, const Bufs
     }
     // moments this lane sums (see the sweep below): rows x, y, z; places of xx, xy, xz, yz among the moments
     const int task = lane & 7, cls = (lane >> 3) & 1, hf = lane >> 4;
-    const int tx = (0x75241630 >> (4 * task)) & 7, ty = (0x72313001 >> (4 * task)) & 7, tz = (0x74665542 >> (4 * task)) & 7;
-    auto place = [](int a, int d) { return a == 7 ? 1 : (a == 6 && d == 6 ? 0 : (a == 6 ? 2 + d : (d == 6 ? 2 + a : 8 + tri(a, d)))); };
-    const int pl_xx = place(tx, tx), pl_xy = place(tx, ty), pl_xz = place(tx, tz), pl_yz = place(ty, tz);
+    const int tx = moment_row_x(task), ty = moment_row_y(task), tz = moment_row_z(task);
+    const int pl_xx = moment_place(tx, tx), pl_xy = moment_place(tx, ty), pl_xz = moment_place(tx, tz), pl_yz = moment_place(ty, tz);
 
     const int nW = G > gw ? (G - gw + nwp - 1) / nwp : 0;   // this warp's Gaussians
     for (int k0 = 0; k0 < nW; k0 += kQuadSlots) {

@@ -167,9 +167,9 @@ __global__ void k_predict_parents(__grid_constant__ const Params prm, double* ex
 // the counter-based stream; non-detection cloud: loaded), predicted, transformed,
 // and staged in the warp's shared-memory rows with its weight w'_s = omega_s pD_s as
 // r d, r and w', where d = y - shift (shift: the Gaussian's first sample, if finite)
-// and r = sqrt(w').  The 29 moments are then summed lane by lane, one product of two
-// rows each (lane q owns moment q: S0 = sum r r, S2 = sum w' w', S1 = sum r (r d),
-// SS = sum (r d)(r d)'), so no per-lane accumulators live through the sample loop.
+// and r = sqrt(w').  The 29 moments (S0 = sum r r, S2 = sum w' w', S1 = sum r (r d),
+// SS = sum (r d)(r d)') are then summed from the rows, four products of three rows and
+// every fourth sample a lane, so no per-lane accumulators live through the sample loop.
 // With the reference's normalised weights w'_s / S0, mean = shift + S1/S0 and the
 // weighted covariance is (SS/S0 - d d') (1 + S2/S0^2), d = S1/S0 (the (W^2 + SS)/W
 // normaliser of kernels.cu:196 with W = 1).  Zero-weight samples do not enter the sums
@@ -211,59 +211,27 @@ __device__ __forceinline__ void ltz_plus_mean(const double* line, const double z
     ltz_line<double, double2, 2>(line, z, y);
 }
 
-// sum over the samples of a[s] b[s], four partial sums over 4-sample pieces read in
-// 16 bytes (row starts are 16-byte aligned): first the nt pieces of the tail rows (ta,
-// tb), then pieces i0 .. n4-1 of the main rows (a, b) -- the order of one sweep over
-// rows holding all samples, so the sums do not depend on where samples were staged
-// FP32: the partial sums run in pairs through sm_100's packed multiply-add (fma.rn.f32x2:
-// two independent single-precision fused multiply-adds, each rounded as fma.rn.f32), two
-// instructions per piece instead of four, with the same results
 __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
     unsigned long long d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
     return d;
 }
-__device__ __forceinline__ float moment_sweep(const float* ta, const float* tb, int nt, const float* a,
-                                              const float* b, int i0, int n4) {
-    unsigned long long s01 = 0ull, s23 = 0ull;   // (s0, s1) and (s2, s3), both +0.0f
-    auto piece = [&](const float4 y, const float4 z) {
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s01) : "l"(pack_f32x2(y.x, y.y)), "l"(pack_f32x2(z.x, z.y)));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s23) : "l"(pack_f32x2(y.z, y.w)), "l"(pack_f32x2(z.z, z.w)));
-    };
-    for (int i = 0; i < nt; ++i) piece(reinterpret_cast<const float4*>(ta)[i], reinterpret_cast<const float4*>(tb)[i]);
-    for (int i = i0; i < n4; ++i) piece(reinterpret_cast<const float4*>(a)[i], reinterpret_cast<const float4*>(b)[i]);
-    float s0, s1, s2, s3;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(s01));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(s2), "=f"(s3) : "l"(s23));
-    return (s0 + s1) + (s2 + s3);
-}
-__device__ __forceinline__ double moment_sweep(const double* ta, const double* tb, int nt, const double* a,
-                                               const double* b, int i0, int n4) {
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    auto piece = [&](const double* y, const double* z) {
-        const double2 y0 = reinterpret_cast<const double2*>(y)[0], z0 = reinterpret_cast<const double2*>(z)[0];
-        const double2 y1 = reinterpret_cast<const double2*>(y)[1], z1 = reinterpret_cast<const double2*>(z)[1];
-        s0 += y0.x * z0.x;
-        s1 += y0.y * z0.y;
-        s2 += y1.x * z1.x;
-        s3 += y1.y * z1.y;
-    };
-    for (int i = 0; i < nt; ++i) piece(ta + 4 * i, tb + 4 * i);
-    for (int i = i0; i < n4; ++i) piece(a + 4 * i, b + 4 * i);
-    return (s0 + s1) + (s2 + s3);
-}
 
-// Sample layout.  A warp takes its Gaussians (j = warp, warp + 8, ...) in rounds of up
-// to 8.  With R = P mod 32 in {4, 8, 16} (P = 100: R = 4), samples [0, R) of the
-// round's 32 / R Gaussians fill one tail pass (lane = Gaussian * R + sample) and
-// samples [R, P) of each Gaussian fill whole warp passes (lane l: R + 32 t + l); with
-// any other R every sample is taken in warp passes.  So a pass has no idle lanes when
-// P = 32 m + R, and lanes of one pass share a Gaussian (no divergence) outside the
-// tail pass.  Staged rows per warp: 8 main rows of sY values (r d[6], r, w' at sample
-// index) and a tail block of 9 R values per Gaussian (the same 8 rows of R samples):
-// sY puts the eight rows a lane-per-moment sweep reads at one sample index (16-byte
-// pieces) in distinct banks, and the 9 R tail stride does the same for the tail
-// pass's stores (lanes of distinct Gaussians, same sample).
+// Sample layout.  A warp takes its Gaussians in rounds of up to 8.  With R = P mod 32 in
+// {4, 8, 16} (P = 100: R = 4), samples [0, R) of the round's 32 / R Gaussians fill one
+// tail pass (lane = Gaussian * R + sample) and samples [R, P) of each Gaussian fill whole
+// warp passes (lane l: R + 32 t + l); with any other R every sample is taken in warp
+// passes.  So a pass has no idle lanes when P = 32 m + R, and lanes of one pass share a
+// Gaussian (no divergence) outside the tail pass.  Staged rows per warp: 8 main rows of sY
+// values (r d[6], r, w' at sample index) and 8 tail rows; the strides put the rows that
+// the sweep reads at one sample index in distinct banks.
+// In FP64 (k_cloud_fit's use; the fused update's in both precisions) what bounds it is
+// issue (0.68 per scheduler and cycle, a quarter of it constants of the logarithm, root,
+// sine and cosine, with the FP64 pipe at 44 %).  Blocks of 4 warps and 96 registers, five
+// to an SM, with one copy of the sampling code: 5.37 -> 5.07 ms for 4096 parents x 256
+// Gaussians x 100 samples (two blocks of 8 warps at 126 registers and three copies
+// before); the products of a lane's three rows cut the sweep's shared-memory reads from
+// 400 to 150 cycles per Gaussian.
 template <typename T> __host__ __device__ constexpr int stage_stride(int P4) {
     return sizeof(T) == 4 ? ((P4 % 8 == 4) ? P4 : P4 + 4) : P4 + 2;
 }
@@ -274,13 +242,31 @@ __host__ __device__ constexpr int fit_tail(int P) {
 template <typename T> __host__ __device__ constexpr int cloud_stride(int P) {
     return sizeof(T) == 4 ? ((P + 7) & ~7) : ((P + 3) & ~3);
 }
-constexpr int kFitWarps = 8;
+constexpr int kFitWarps = 4;     // warps of a k_cloud_fit block in FP64
 constexpr int kFitRound = 8;     // Gaussians per warp and round
 constexpr int kStageRows = 8;    // r d[6], r, w'
-constexpr int kTailFloats = 288; // 32 / R Gaussians x 9 R per warp
-template <typename T> __host__ __device__ inline size_t cloud_fit_smem_bytes(int P) {
-    const int P4 = (P + 3) & ~3;
-    return (size_t)kFitWarps * (kStageRows * stage_stride<T>(P4) + kTailFloats) * sizeof(T);
+// The tail pass's staged rows: sample s of Gaussian gi at column gi R + s, at most 32; 34 is 16
+// bytes times an odd number in FP64 (and spreads FP32 words)
+constexpr int kTailStride = 34;
+constexpr int kTailFloats = kStageRows * kTailStride;
+// The sweep's rows: eight tasks of three rows x, y, z each; the first seven are the lines of
+// the Fano plane on the rows r d[6], r, so that the products xx, xy, xz, yz hold every product
+// of two of them once; the eighth sums w'w'.  moment_place: 0 sum r r, 1 sum w'w', 2-7 sum
+// r (r d), 8-28 sum (r d)(r d)'.
+__device__ __forceinline__ int moment_row_x(int t) { return (0x75241630 >> (4 * t)) & 7; }
+__device__ __forceinline__ int moment_row_y(int t) { return (0x72313001 >> (4 * t)) & 7; }
+__device__ __forceinline__ int moment_row_z(int t) { return (0x74665542 >> (4 * t)) & 7; }
+__device__ __forceinline__ int moment_place(int a, int b) {
+    return a == 7 ? 1 : (a == 6 && b == 6 ? 0 : (a == 6 ? 2 + b : (b == 6 ? 2 + a : 8 + tri(a, b))));
+}
+// per warp, in values: main and tail rows, the round's factors and means (28) and shifts (6)
+template <typename T> __host__ __device__ constexpr int fit_warp_values(int P) {
+    return kStageRows * stage_stride<T>((P + 3) & ~3) + (fit_tail(P) ? kTailFloats : 0) + kFitRound * (28 + 6);
+}
+// the table of mean pD values, n = 0..P
+template <typename T> __host__ __device__ constexpr int fit_pbar_values(int P) { return (P + 4) & ~3; }
+template <typename T> __host__ __device__ inline size_t cloud_fit_smem_bytes(int P, int warps) {
+    return (size_t)(fit_pbar_values<T>(P) + warps * fit_warp_values<T>(P)) * sizeof(T);
 }
 
 // PC > 0: the body for exactly PC samples per feature, whose strides, loop bounds and
@@ -305,9 +291,9 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
         }
     }
     // the parent's Gaussians are shared by the warps of its `split` blocks: block c's
-    // warp w takes j = gw, gw + nwp, ... (gw = c * kFitWarps + w, nwp = split * kFitWarps)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gw = c * kFitWarps + warp, nwp = split * kFitWarps;
+    // warp w takes j = gw, gw + nwp, ... (gw = c nw + w, nwp = split nw, nw warps a block)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int gw = c * nw + warp, nwp = split * nw;
     const int row = b.src[p];
     const int G = min(b.map_n[cur][row], prm.Gcap);
     const int P = PC > 0 ? PC : prm.P, Ps = PC > 0 ? cloud_stride<T>(PC) : prm.Ps;
@@ -315,15 +301,15 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
     const int sY = stage_stride<T>(P4);
     const int R = fit_tail(P);                      // tail samples per Gaussian (0: no tail pass)
     const int TG = R ? 32 / R : kFitRound;          // Gaussians per round
-    T* Y = s_stage + (size_t)warp * kStageRows * sY;                                   // main rows
-    T* Yt = s_stage + (size_t)kFitWarps * kStageRows * sY + (size_t)warp * kTailFloats;  // tail blocks
-    __shared__ T s_shift[kFitWarps * kFitRound * 6];          // per warp and Gaussian of the round
-    __shared__ __align__(16) T s_L[kFitWarps * kFitRound * 28];  // Cholesky factor and mean of merged ones
-    __shared__ Pose<T> pose_upd, pose_src;
-    __shared__ int s_rd, s_wr;
     // mean pD of a Gaussian with n of its P samples in view, n = 0..P (P <= 256): the
     // value n pD / P in FP64, rounded to T, looked up instead of divided per Gaussian
-    __shared__ T s_pbar[257];
+    T* s_pbar = s_stage;
+    T* Y = s_stage + fit_pbar_values<T>(P) + (size_t)warp * fit_warp_values<T>(P);   // main rows
+    T* Yt = Y + kStageRows * sY;                                                   // tail rows
+    T* Lw = Yt + (R ? kTailFloats : 0);       // factor and mean of the round's merged Gaussians
+    T* shw = Lw + kFitRound * 28;             // shifts of the round's Gaussians
+    __shared__ Pose<T> pose_upd, pose_src;
+    __shared__ int s_rd, s_wr;
     for (int i = threadIdx.x; i <= P; i += blockDim.x) s_pbar[i] = (T)((double)i * prm.model.pd / (double)P);
     // the two poses (FP64 rotation terms) by threads of two warps, side by side
     if (threadIdx.x == 32) pose_src = make_pose<T>(b.map_ext[cur] + 12 * row);
@@ -347,19 +333,18 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
     const T invP = T(1) / T(P);
     const T dtT = (T)dt, half_dt2 = T(0.5) * (T)dt * (T)dt;
     const T min_w = (T)prm.min_weight;
-    T* shw = s_shift + warp * kFitRound * 6;
-    T* Lw = s_L + warp * kFitRound * 28;
-    // moment owned by this lane: rows (ra, rb) of the product Y[ra] * Y[rb]: lane 0
-    // S0 = sum r r, lane 1 S2 = sum w' w', lanes 2-7 S1 = sum r (r d), lanes 8-28 SS
+    // fitted row element of this lane (W, pD, mean[6], packed cov[21]): lanes 2-7 the mean,
+    // lanes 8-28 the covariance entry (ra, rb)
     int ra = 6, rb = 6;
-    if (lane == 1) ra = rb = 7;
-    else if (lane >= 2 && lane < 8) rb = lane - 2;
-    else if (lane >= 8 && lane < 29) {
+    if (lane >= 8 && lane < 29) {
         int e = lane - 8, aa = 0;
         while ((aa + 1) * (aa + 2) / 2 <= e) ++aa;
         ra = aa;
         rb = e - aa * (aa + 1) / 2;
     }
+    // moments this lane sums (the sweep, below)
+    const int task = lane & 7, cls = lane >> 3;
+    const int tx = moment_row_x(task), ty = moment_row_y(task), tz = moment_row_z(task);
     // one sample s of Gaussian j (entry ref, factor line Lg): the predicted particle X,
     // its measurement y; returns the sample weight omega (1/P for a drawn sample)
     auto sample = [&](int ref, int j, int s, const T* Lg, T (&X)[6], T (&y)[6]) -> T {
@@ -450,15 +435,21 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
         for (int k = 0; k < kFitRound; ++k)
             if (((merged >> k) & 1u) && lane < 28) Lw[k * 28 + lane] = lv[k];
         __syncwarp();
-        // tail pass: samples [0, R) of the round's Gaussians; lane gi * R (sample 0)
-        // gives its Gaussian's shift
-        int t_in = 0;
+        // Passes of the round, one code path for all (three copies of the sampling code, with
+        // their logarithms, roots and sines, missed in the instruction cache): first the tail
+        // pass, samples [0, R) of every Gaussian, lane gi R + s; then, for each Gaussian, whole
+        // warps over samples [R, P4), and the fit.
+        unsigned t_in = 0;             // tail pass: this lane's Gaussian's samples in view
         bool t_any = false;
-        if (R) {
-            const int gi = lane / R, s = lane - gi * R;
-            const bool valid = gi < nR;
+        int k = R ? -1 : 0, s0 = R;    // Gaussian of the round (-1: the tail pass), first sample
+        int n_in = 0;
+        bool any = false, raw = false;
+        while (true) {
+            const int gi = k < 0 ? lane / R : k;
+            const int s = k < 0 ? lane - gi * R : s0 + lane;
+            const bool valid = k < 0 ? gi < nR : s < P;
             const int ref = __shfl_sync(0xffffffffu, my_ref, gi & 31);
-            const bool wnd = __shfl_sync(0xffffffffu, my_W, gi & 31) >= min_w;
+            const T W = __shfl_sync(0xffffffffu, my_W, gi & 31);
             const int j = gw + nwp * (k0 + gi);
             T X[6], y[6], om = 0;
             if (valid) {
@@ -467,102 +458,95 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
 #pragma unroll
                 for (int a2 = 0; a2 < 6; ++a2) { X[a2] = 0; y[a2] = 0; }
             }
-            const bool inr = valid && in_range(y, mt);
-            const T pds = inr ? (T)mt.pd : T(0);
-            if (valid && wnd) write_nd(j, s, X, pds);
-            const T wp = om * pds;
-            T shift[6];
+            if (raw) {   // the unweighted fit's rows: y itself (below)
+                if (s < P4) {
 #pragma unroll
-            for (int a2 = 0; a2 < 6; ++a2) {
-                const T v = __shfl_sync(0xffffffffu, y[a2], lane - s);
-                shift[a2] = isfinite(v) ? v : T(0);
-            }
-            if (valid && s == 0) {
-#pragma unroll
-                for (int a2 = 0; a2 < 6; ++a2) shw[gi * 6 + a2] = shift[a2];
-            }
-            stage(Yt + gi * 9 * R + s, R, y, shift, wp);
-            const unsigned gm = (R == 32 ? 0xffffffffu : ((1u << R) - 1u)) << (gi * R & 31);
-            t_in = __popc(__ballot_sync(0xffffffffu, inr) & gm);
-            t_any = (__ballot_sync(0xffffffffu, wp != T(0)) & gm) != 0u;
-        }
-        __syncwarp();
-        for (int k = 0; k < nR; ++k) {
-            const int j = gw + nwp * (k0 + k);
-            const int ref = __shfl_sync(0xffffffffu, my_ref, k);
-            const T W = __shfl_sync(0xffffffffu, my_W, k);
-            const bool wnd = W >= min_w;
-            const T* Lg = Lw + k * 28;
-            const T* Ytk = Yt + k * 9 * R;
-            T shift[6];
-            if (R) {
-#pragma unroll
-                for (int a2 = 0; a2 < 6; ++a2) shift[a2] = shw[k * 6 + a2];
-            }
-            int n_in = R ? __shfl_sync(0xffffffffu, t_in, (k * R) & 31) : 0;
-            bool any = R ? __shfl_sync(0xffffffffu, (int)t_any, (k * R) & 31) != 0 : false;
-            // warp passes over samples [R, P4): moment rows, non-detection clouds
-            for (int s0 = R; s0 < P4; s0 += 32) {
-                const int s = s0 + lane;
-                const bool valid = s < P;
-                T X[6], y[6], om = 0;
-                if (valid) {
-                    om = sample(ref, j, s, Lg, X, y);
-                } else {
-#pragma unroll
-                    for (int a2 = 0; a2 < 6; ++a2) { X[a2] = 0; y[a2] = 0; }
+                    for (int a2 = 0; a2 < 6; ++a2) Y[a2 * sY + s] = y[a2];
                 }
+            } else {
                 const bool inr = valid && in_range(y, mt);
                 const T pds = inr ? (T)mt.pd : T(0);
-                n_in += __popc(__ballot_sync(0xffffffffu, inr));
-                if (valid && wnd) write_nd(j, s, X, pds);
+                if (valid && W >= min_w) write_nd(j, s, X, pds);
                 const T wp = om * pds;
-                any |= __any_sync(0xffffffffu, wp != T(0));
-                if (!R && s0 == 0) {   // shift: the Gaussian's first sample, if finite, else 0
-#pragma unroll
-                    for (int a2 = 0; a2 < 6; ++a2) {
-                        const T v = __shfl_sync(0xffffffffu, y[a2], 0);
-                        shift[a2] = isfinite(v) ? v : T(0);
-                    }
-                    if (lane < 6) {   // static indices: the shift stays in registers
-#pragma unroll
-                        for (int a2 = 0; a2 < 6; ++a2)
-                            if (lane == a2) shw[k * 6 + a2] = shift[a2];
-                    }
+                const unsigned b_in = __ballot_sync(0xffffffffu, inr), b_nz = __ballot_sync(0xffffffffu, wp != T(0));
+                if (k < 0) {
+                    const unsigned gm = ((1u << R) - 1u) << (gi * R & 31);
+                    t_in = __popc(b_in & gm);
+                    t_any = (b_nz & gm) != 0u;
+                } else {
+                    n_in += __popc(b_in);
+                    any |= b_nz != 0u;
                 }
-                if (s < P4) stage(Y + s, sY, y, shift, wp);
-            }
-            const T pbar = s_pbar[n_in];
-            const bool raw = !any && n_in > 0 && m.pd > 0.0;
-            if (raw) {
-                // the fallback fit (below) needs the raw samples: rare, so they are drawn
-                // again, every sample in warp passes, y itself staged in the main rows
+                // the shift: the Gaussian's first sample, if finite, else 0
+                if (valid && s == 0) {
+#pragma unroll
+                    for (int a2 = 0; a2 < 6; ++a2) shw[gi * 6 + a2] = isfinite(y[a2]) ? y[a2] : T(0);
+                }
                 __syncwarp();
-                for (int s0 = 0; s0 < P4; s0 += 32) {
-                    const int s = s0 + lane;
-                    T X[6], y[6];
-                    if (s < P) {
-                        sample(ref, j, s, Lg, X, y);
-                    } else {
+                T shift[6];
 #pragma unroll
-                        for (int a2 = 0; a2 < 6; ++a2) y[a2] = 0;
-                    }
-                    if (s < P4) {
-#pragma unroll
-                        for (int a2 = 0; a2 < 6; ++a2) Y[a2 * sY + s] = y[a2];
-                    }
-                }
+                for (int a2 = 0; a2 < 6; ++a2) shift[a2] = shw[(k < 0 ? gi % TG : k) * 6 + a2];
+                if (k < 0) stage(Yt + gi * R + s, kTailStride, y, shift, wp);
+                else if (s < P4) stage(Y + s, sY, y, shift, wp);
             }
             __syncwarp();
+            if (k < 0) {
+                k = 0;
+                n_in = __shfl_sync(0xffffffffu, (int)t_in, 0);
+                any = __shfl_sync(0xffffffffu, (int)t_any, 0) != 0;
+                if (R < P4) continue;
+            } else {
+                s0 += 32;
+                if (s0 < P4) continue;
+            }
+            const T pbar = s_pbar[n_in];
+            if (!raw && !any && n_in > 0 && m.pd > 0.0) {
+                // the unweighted fit needs the raw samples: rare, so they are drawn again
+                raw = true;
+                s0 = 0;
+                continue;
+            }
             const T* sh = shw + k * 6;
-            // fitted row element `lane` (W, pD, mean[6], packed cov[21]), written from registers
-            T fv = lane == 0 ? W : pbar;
+            // fitted row element `lane`, written from registers
+            const T Wk = __shfl_sync(0xffffffffu, my_W, k);
+            T fv = lane == 0 ? Wk : pbar;
             if (any) {
-                // lane q < 29: moment q over the samples, four partial sums
-                const T mom = lane < 29 ? moment_sweep(Ytk + ra * R, Ytk + rb * R, R / 4, Y + ra * sY, Y + rb * sY,
-                                                       R / 4, P4 / 4)
-                                        : T(0);
-                const T S0 = __shfl_sync(0xffffffffu, mom, 0), S2 = __shfl_sync(0xffffffffu, mom, 1);
+                // the sweep: lane 8 c + t sums the products xx, xy, xz, yz of three staged rows over
+                // the samples s = c mod 4 (the four partial sums of a moment, in sample order)
+                T xx = 0, xy = 0, xz = 0, yz = 0;
+                auto run = [&](const T* base, int stride, int from, int to) {
+                    const T *px = base + tx * stride + cls, *py = base + ty * stride + cls, *pz = base + tz * stride + cls;
+#pragma unroll 4
+                    for (int i = from; i < to; ++i) {
+                        const T vx = px[4 * i], vy = py[4 * i], vz = pz[4 * i];
+                        xx += vx * vx;
+                        xy += vx * vy;
+                        xz += vx * vz;
+                        yz += vy * vz;
+                    }
+                };
+                run(Yt + k * R, kTailStride, 0, R / 4);
+                run(Y, sY, R / 4, P4 / 4);
+#pragma unroll
+                for (int o = 8; o < 32; o <<= 1) {
+                    xx += __shfl_xor_sync(0xffffffffu, xx, o);
+                    xy += __shfl_xor_sync(0xffffffffu, xy, o);
+                    xz += __shfl_xor_sync(0xffffffffu, xz, o);
+                    yz += __shfl_xor_sync(0xffffffffu, yz, o);
+                }
+                __syncwarp();   // every row is read: the moments go where the first rows were
+                T* mo = Y;
+                if (cls == 0) {
+                    mo[moment_place(tx, tx)] = xx;
+                    if (task != 7) {
+                        mo[moment_place(tx, ty)] = xy;
+                        mo[moment_place(tx, tz)] = xz;
+                        mo[moment_place(ty, tz)] = yz;
+                    }
+                }
+                __syncwarp();
+                const T mom = lane < 29 ? mo[lane] : T(0);
+                const T S0 = mo[0], S2 = mo[1];
                 const T inv = T(1) / S0, scale = T(1) + S2 * inv * inv;
                 // lanes 2-7 hold S1 (the mean offsets), lanes 8-28 hold SS
                 const T dl = (lane >= 2 && lane < 8) ? mom * inv : T(0);
@@ -582,7 +566,7 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
                 // samples) and covariance x (P + P)/P over the valid samples (raw rows)
                 T mu = 0;
                 if (lane < 6) {
-                    for (int s = 0; s < P; ++s) mu += Y[lane * sY + s];
+                    for (int i = 0; i < P; ++i) mu += Y[lane * sY + i];
                 }
                 T mus[6];
 #pragma unroll
@@ -595,7 +579,7 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
                         if (ra == a2) ma = mus[a2];
                         if (rb == a2) mb = mus[a2];
                     }
-                    for (int s = 0; s < P; ++s) cva += (Y[ra * sY + s] - ma) * (Y[rb * sY + s] - mb);
+                    for (int i = 0; i < P; ++i) cva += (Y[ra * sY + i] - ma) * (Y[rb * sY + i] - mb);
                 }
                 const T scale = (T(P) * T(P) + T(P)) / T(P);
                 const T mu_e = __shfl_sync(0xffffffffu, mu, (lane - 2) & 31);   // mean element lane - 2
@@ -606,9 +590,14 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
                 if (lane >= 2 && lane < 8) fv = sh[lane - 2];
                 if (lane >= 8) fv = T(0);
             }
-            T* fr = b.fit + ((size_t)p * prm.Gcap + j) * kRow;
+            T* fr = b.fit + ((size_t)p * prm.Gcap + gw + nwp * (k0 + k)) * kRow;
             if (lane < 29) fr[lane] = fv;
-            __syncwarp();   // the sweep's reads of the rows end before the next Gaussian's staging
+            __syncwarp();   // the rows' reads end before the next Gaussian's staging
+            if (++k >= nR) break;
+            s0 = R;
+            raw = false;
+            n_in = R ? __shfl_sync(0xffffffffu, (int)t_in, (k * R) & 31) : 0;
+            any = R ? __shfl_sync(0xffffffffu, (int)t_any, (k * R) & 31) != 0 : false;
         }
     }
     __syncthreads();
@@ -637,9 +626,9 @@ __device__ __forceinline__ void cloud_fit_any(const Params& prm, const Bufs<T>& 
 }
 // threads of a cloud-fit block, and blocks an SM is to hold
 template <typename T> constexpr int kFitThreads = 32 * (sizeof(T) == 4 ? kQuadWarps : kFitWarps);
-template <typename T> constexpr int kFitBlocks = sizeof(T) == 4 ? 4 : 2;
+template <typename T> constexpr int kFitBlocks = sizeof(T) == 4 ? 4 : 5;
 template <typename T> __host__ __device__ inline size_t fit_kernel_smem_bytes(int P) {
-    return sizeof(T) == 4 ? quad_fit_smem_bytes(P) : cloud_fit_smem_bytes<T>(P);
+    return sizeof(T) == 4 ? quad_fit_smem_bytes(P) : cloud_fit_smem_bytes<T>(P, kFitWarps);
 }
 
 // grid: `split` blocks per parent (block x: parent x / split, part x % split)
@@ -2065,7 +2054,7 @@ __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
 // order, and the merge sorts them).
 constexpr int kFusedThreads = 256;
 template <typename T> inline size_t fused_smem_bytes(int P, int Gcap, int Scap) {
-    size_t s = cloud_fit_smem_bytes<T>(P);
+    size_t s = cloud_fit_smem_bytes<T>(P, kFusedThreads / 32);
     const size_t cand[3] = {prep_smem_bytes<T>(), likelihood_smem_bytes<T>(Gcap, kFusedThreads),
                             merge_shared_bytes<T>(Scap, Gcap, kFusedThreads / 32)};
     for (size_t c : cand) s = c > s ? c : s;
