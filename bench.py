@@ -534,7 +534,7 @@ def extra_workloads(args, pkg):
 def run_batched(args, pkg, quiet=False):
     """Many-filter workload: 64 filters of uneven size (batched_specs), grouped into
     device-resident waves under an 80% HBM budget.  Each wave is one SCPHDBatch
-    stepped from a captured CUDA graph (seven kernels per frame for all its filters).
+    stepped from a captured CUDA graph (six kernels per frame for all its filters).
     Timed per wave: K pairs of batched frames alternating with K pairs of frames in
     which the same filters are stepped plain, one filter at a time (device events on
     the batch stream), then K batched frames end to end from host arrays with the
@@ -612,7 +612,7 @@ def run_batched(args, pkg, quiet=False):
                 if form == "b":
                     res["frame_ms"] += [e[0].elapsed_time(e[1]), e[1].elapsed_time(e[2])]
                     res["truncations"] += sum(int(b[0] - a[0]) for a, b in zip(c0, c1))
-                    lb += 14   # seven kernels per batched frame, two frames
+                    lb += 12   # six kernels per batched frame, two frames
         res["launches"] += lb
         res["overflows"] += sum(int(f.counters()[1]) for f in fs)
         # end to end: host frames in, parent states out, through the public API.  The

@@ -281,10 +281,10 @@ scphd_status scphd_device_bytes(const scphd_config* cfg, int64_t* bytes);
 
 /* ------------------------------------------------------------------ batches
  * Many filters advanced together: every batched step runs predict(dt) + update +
- * resample for all member filters with one kernel launch per stage (seven per frame,
- * or four with the fused update, whatever the number of filters; one more where
- * max_survivors is large, for the parents with more survivors than most), each launch
- * covering every filter's parents
+ * resample for all member filters with six kernel launches per frame (three with the
+ * fused update), whatever the number of filters, and one more where max_survivors is
+ * large, for the parents with more survivors than most; each launch covers every
+ * filter's parents
  * through a block -> (filter, parent) map.  Member filters must share device,
  * precision and meas_dim; they may differ in size.  While in a batch, the filters
  * issue all their work on the batch's stream (their own stream is restored by
@@ -318,8 +318,8 @@ scphd_status scphd_batch_step_device(scphd_batch* b, double dt, const scphd_fram
 void* scphd_batch_stream(scphd_batch* b);
 /* The batch's update path, as scphd_set_fused / scphd_get_fused: 0 (default) the
  * stage kernels, 1 the fused kernel (set before the first graph capture).  A fused
- * batch step is four launches per group of up to 32 filters: prediction (with the
- * frame's measurement conversion), the fused update, parent weights, resampling. */
+ * batch step is three launches per group of up to 32 filters: prediction (with the
+ * frame's measurement conversion), the fused update, parent weights with resampling. */
 scphd_status scphd_batch_set_fused(scphd_batch* b, int32_t mode);
 scphd_status scphd_batch_get_fused(scphd_batch* b, int32_t* fused);
 /* The batch's cloud-fit tiling, as scphd_set_fit_split / scphd_get_fit_split (one

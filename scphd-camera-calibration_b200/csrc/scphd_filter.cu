@@ -209,7 +209,7 @@ struct scphd_filter {
     }
     virtual scphd_status init() = 0;
     virtual scphd_status predict(double dt) = 0;
-    virtual scphd_status update_staged(int M, int fixed) = 0;
+    virtual scphd_status update_staged(int M, int fixed, bool then_resample) = 0;
     virtual scphd_status resample(int32_t* resampled, bool read_back) = 0;
     virtual scphd_status get_particles(double* st, double* lw) = 0;
     virtual scphd_status get_particles_async(double* st, double* lw) = 0;
@@ -241,7 +241,7 @@ template <typename T> class Filter final : public scphd_filter {
 public:
     Bufs<T> b{};
     void* arena_ptr = nullptr;
-    T* dump = nullptr;        // Gcap x 7 x Ps cloud dump scratch
+    double* dump = nullptr;   // Gcap x 7 x P: a parent's cloud for the host
     size_t merge_smem = 0;       // the full survivor capacity's
     int merge_over_grid = 0;     // blocks of the second merge launch
     struct MergeLaunch { int S = 0; size_t smem = 0; } merge_at[2];   // first launch: kMergeThreads, 128 threads
@@ -288,7 +288,8 @@ public:
         b.flags = a.take<int>(4);
         b.resample_idx = a.take<int>(N);
         b.counters = a.take<unsigned long long>(16);
-        dump = a.take<T>(G * 7 * Ps);
+        b.snap = a.take<unsigned long long>(2);
+        dump = a.take<double>(G * 7 * prm.P);
         b.fit_n = a.take<int>(N);
         d_stage = a.take<double>(Mc * 3);
     }
@@ -382,7 +383,7 @@ public:
     scphd_status materialize_pending() {
         const int N = prm.N;
         k_materialize<T><<<N, 256, 0, stream>>>(prm, b, cur, b.cloud[cur ^ 1], b.map[cur ^ 1], b.map_ref[cur ^ 1],
-                                                 b.map_n[cur ^ 1], 1, pending_dt, pending_frame, sample_frame[cur], -1);
+                                                 b.map_n[cur ^ 1], 1, pending_dt, pending_frame, sample_frame[cur]);
         LAUNCHED();
         cur ^= 1;
         k_reset_src<<<(N + 255) / 256, 256, 0, stream>>>(b.src, N);
@@ -409,7 +410,8 @@ public:
         return SCPHD_OK;
     }
 
-    template <int K> scphd_status update_k(int M, int fixed) {
+    // then_resample: the step's resampling follows in the same launch as the weights
+    template <int K> scphd_status update_k(int M, int fixed, bool then_resample) {
         const int N = prm.N;
         {
             const scphd_status ts = tune_collect();
@@ -420,14 +422,13 @@ public:
         if (timed) CUDA_TRY(cudaEventRecord(tune_ev[0], stream));
         if (fused_next()) {
             k_stage_frame<T, K><<<1, 256, 0, stream>>>(b.z, M > 0 ? d_stage : nullptr, M > 0 ? d_stage + M : nullptr,
-                                                       M > 0 ? d_stage + 2 * M : nullptr, M, b.counters, b.flags + 2);
+                                                       M > 0 ? d_stage + 2 * M : nullptr, M, b.flags + 2);
             LAUNCHED();
             const FrameArgs fa{cur, M, fixed, pending ? 1 : 0, pending_dt, pending_frame, sample_frame[cur], frame,
                                nullptr, nullptr, nullptr};
             k_fused<T, K><<<fused_grid, kFusedThreads, fused_smem, stream>>>(prm, b, fa, b.flags + 2);
             LAUNCHED();
         } else {
-            CUDA_TRY(cudaMemsetAsync(b.counters + 4, 0, 2 * sizeof(unsigned long long), stream));
             int h = stage_begin(1);
             const double* zs[3] = {M > 0 ? d_stage : nullptr, M > 0 ? d_stage + M : nullptr,
                                    M > 0 ? d_stage + 2 * M : nullptr};
@@ -477,7 +478,12 @@ public:
             tune_pending = tune_trials % kShapes;
         }
         int h = stage_begin(4);
-        k_weights<<<1, 1024, 0, stream>>>(N, b.lw, b.loglik, fixed ? 0 : 1, b.scal, b.counters);
+        if (then_resample) {
+            k_weights_resample<T><<<1, weights_threads(N), 0, stream>>>(prm, b, fixed ? 0 : 1, frame);
+            LAUNCHED();
+            return gather_parents();
+        }
+        k_weights<T><<<1, weights_threads(N), 0, stream>>>(b, N, fixed ? 0 : 1);
         LAUNCHED();
         stage_end(h);
         return SCPHD_OK;
@@ -485,8 +491,8 @@ public:
 
     // one update: the kernels convert the staged measurements, record the fitted
     // counts, reset the src indirection and count the frame themselves
-    scphd_status update_staged(int M, int fixed) override {
-        scphd_status s = prm.K == 2 ? update_k<2>(M, fixed) : update_k<3>(M, fixed);
+    scphd_status update_staged(int M, int fixed, bool then_resample) override {
+        scphd_status s = prm.K == 2 ? update_k<2>(M, fixed, then_resample) : update_k<3>(M, fixed, then_resample);
         if (s != SCPHD_OK) return s;
         cur ^= 1;
         sample_frame[cur] = frame;
@@ -494,16 +500,25 @@ public:
         return SCPHD_OK;
     }
 
-    scphd_status resample(int32_t* resampled, bool read_back) override {
-        int h = stage_begin(5);
-        k_resample<<<1, 1024, 0, stream>>>(prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal, b.flags,
-                                           b.resample_idx, frame, 0, -1.0, b.counters, 0);
-        LAUNCHED();
+    // the resampled parents' states, where the resampling block left them (resample_body)
+    scphd_status gather_parents() {
+        if (prm.N <= kGatherParents) return SCPHD_OK;
         const int ng = (12 * prm.N + 255) / 256;
         k_gather_parents<<<ng, 256, 0, stream>>>(b.flags, b.resample_idx, b.ext, b.ext_tmp, prm.N);
         LAUNCHED();
         k_copy_parents<<<ng, 256, 0, stream>>>(b.flags, b.ext_tmp, b.ext, prm.N);
         LAUNCHED();
+        return SCPHD_OK;
+    }
+
+    scphd_status resample(int32_t* resampled, bool read_back) override {
+        int h = stage_begin(5);
+        k_resample<<<1, weights_threads(prm.N), 0, stream>>>(prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal,
+                                                             b.flags, b.resample_idx, frame, 0, -1.0, b.counters,
+                                                             prm.N <= kGatherParents);
+        LAUNCHED();
+        const scphd_status gs = gather_parents();
+        if (gs != SCPHD_OK) return gs;
         stage_end(h);
         if (read_back) {
             int f = 0;
@@ -563,20 +578,15 @@ public:
         std::vector<int> src, n;
         scphd_status s = host_rows(src, n);
         if (s != SCPHD_OK) return s;
-        const int G = n[src[p]], P = prm.P, Ps = prm.Ps;
+        const int G = n[src[p]], P = prm.P;
         if (G == 0) return SCPHD_OK;
-        k_materialize<T><<<1, 256, 0, stream>>>(prm, b, cur, dump, nullptr, nullptr, nullptr, pending ? 1 : 0,
-                                                 pending_dt, pending_frame, sample_frame[cur], p);
+        double* d_om = dump + (size_t)G * 6 * P;
+        k_map_cloud<T><<<(G * P + 127) / 128, 128, 0, stream>>>(prm, b, cur, dump, d_om, G, pending ? 1 : 0, pending_dt,
+                                                                pending_frame, sample_frame[cur], p);
         LAUNCHED();
-        std::vector<T> h((size_t)G * 7 * Ps);
-        CUDA_TRY(cudaMemcpyAsync(h.data(), dump, sizeof(T) * h.size(), cudaMemcpyDeviceToHost, stream));
+        if (xyz) CUDA_TRY(cudaMemcpyAsync(xyz, dump, sizeof(double) * G * 6 * P, cudaMemcpyDeviceToHost, stream));
+        if (om) CUDA_TRY(cudaMemcpyAsync(om, d_om, sizeof(double) * G * P, cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
-        for (int j = 0; j < G; ++j)
-            for (int s2 = 0; s2 < P; ++s2) {
-                for (int a = 0; a < 6; ++a)
-                    if (xyz) xyz[((size_t)j * 6 + a) * P + s2] = (double)h[((size_t)j * 7 + a) * Ps + s2];
-                if (om) om[(size_t)j * P + s2] = (double)h[((size_t)j * 7 + 6) * Ps + s2];
-            }
         return SCPHD_OK;
     }
 
@@ -854,7 +864,7 @@ scphd_status scphd_update(scphd_filter* f, const double* u, const double* v, con
     HANDLE(f);
     scphd_status s = stage_host(f, u, v, d, n);
     if (s != SCPHD_OK) return s;
-    return f->update_staged(n, fixed_camera ? 1 : 0);
+    return f->update_staged(n, fixed_camera ? 1 : 0, false);
 }
 
 scphd_status scphd_update_device(scphd_filter* f, const double* u, const double* v, const double* d, int32_t n,
@@ -868,7 +878,7 @@ scphd_status scphd_update_device(scphd_filter* f, const double* u, const double*
         CUDA_TRY(cudaMemcpyAsync(f->d_stage + n, v, sizeof(double) * n, cudaMemcpyDeviceToDevice, f->stream));
         if (d) CUDA_TRY(cudaMemcpyAsync(f->d_stage + 2 * n, d, sizeof(double) * n, cudaMemcpyDeviceToDevice, f->stream));
     }
-    return f->update_staged(n, fixed_camera ? 1 : 0);
+    return f->update_staged(n, fixed_camera ? 1 : 0, false);
 }
 
 scphd_status scphd_resample(scphd_filter* f, int32_t* resampled) {
@@ -884,7 +894,8 @@ scphd_status scphd_step(scphd_filter* f, double dt, const double* u, const doubl
     if (s != SCPHD_OK) return s;
     s = f->predict(dt);
     if (s != SCPHD_OK) return s;
-    s = f->update_staged(n, fixed_camera ? 1 : 0);
+    if (!f->profiling) return f->update_staged(n, fixed_camera ? 1 : 0, true);
+    s = f->update_staged(n, fixed_camera ? 1 : 0, false);   // each stage timed by itself
     if (s != SCPHD_OK) return s;
     return f->resample(nullptr, false);
 }
@@ -903,7 +914,8 @@ scphd_status scphd_step_device(scphd_filter* f, double dt, const double* u, cons
     }
     scphd_status s = f->predict(dt);
     if (s != SCPHD_OK) return s;
-    s = f->update_staged(n, fixed_camera ? 1 : 0);
+    if (!f->profiling) return f->update_staged(n, fixed_camera ? 1 : 0, true);
+    s = f->update_staged(n, fixed_camera ? 1 : 0, false);   // each stage timed by itself
     if (s != SCPHD_OK) return s;
     return f->resample(nullptr, false);
 }
@@ -1306,8 +1318,9 @@ namespace {
 
 template <typename T> struct Batch final : scphd_batch {
     // Filters are launched in groups of up to kBatchSlots, each group with its own
-    // parameter table and block maps; per group and frame seven launches (one kernel
-    // per stage) or four (prediction, the fused update, weights, resampling).
+    // parameter table and block maps; per group and frame six launches (prediction,
+    // cloud fit, Kalman terms, likelihood, merge, weights with resampling; a seventh where
+    // merge_over is set) or three (prediction, the fused update, weights with resampling).
     struct Group {
         int first = 0, count = 0;       // filters [first, first + count)
         SlotTable<T>* tab = nullptr;    // host copy, passed by value at each launch
@@ -1557,11 +1570,7 @@ template <typename T> struct Batch final : scphd_batch {
             }
         }
         for (const Group& g : groups) {
-            k_weights_batch<T><<<g.count, 1024, 0, stream>>>(*g.tab, d_fa + g.first);
-            LAUNCHED();
-        }
-        for (const Group& g : groups) {
-            k_resample_batch<T><<<g.count, 1024, 0, stream>>>(*g.tab, d_fa + g.first);
+            k_weights_resample_batch<T><<<g.count, 1024, 0, stream>>>(*g.tab, d_fa + g.first);
             LAUNCHED();
         }
         if (timed) {
@@ -1573,7 +1582,7 @@ template <typename T> struct Batch final : scphd_batch {
 
     int launches_per_frame() const {
         int n = 0;
-        for (const Group& g : groups) n += path_now() == 2 ? 4 : 7 + (g.merge_over > 0);
+        for (const Group& g : groups) n += path_now() == 2 ? 3 : 6 + (g.merge_over > 0);
         return n;
     }
 

@@ -342,7 +342,6 @@ __device__ __forceinline__ void cloud_fit_f32_body(const Params& prm, const Bufs
         for (int i = 0; i < 3; ++i) tab.upd_t[i] = f2_dup(-pu.t[i]);
         if (c == 0) {
             b.surv_n[p] = 0;
-            atomicAdd(&b.counters[4], (unsigned long long)G * (unsigned long long)M);
             atomicAdd(&b.counters[6], (unsigned long long)G * (unsigned long long)M);
             atomicAdd(&b.counters[10], (unsigned long long)G);
         }

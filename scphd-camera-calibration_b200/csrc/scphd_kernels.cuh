@@ -17,6 +17,7 @@
 //                           clouds, parent log-likelihood               [N CTAs]
 //   k_weights           FP64 log-domain parent weight update + N_eff   [1 CTA]
 //   k_resample          (e) FP64 block scan + systematic resampling     [1 CTA]
+//                       (one launch, k_weights_resample, in a step)
 #pragma once
 
 #include "scphd_device.cuh"
@@ -77,6 +78,7 @@ template <typename T> struct Bufs {
     int* flags;         // [0] resampled, [2] fused work counter, [3] parents listed for the second merge launch
     int* resample_idx;  // N
     unsigned long long* counters;   // 16
+    unsigned long long* snap;       // counters [6], [7] as the last update left them
     int* fit_n;         // N: Gaussians the last update fitted (prior map size)
 };
 
@@ -319,7 +321,6 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
         pose_upd = make_pose<T>(fixed ? zero : b.ext + 12 * p);
         if (c == 0) {
             b.surv_n[p] = 0;
-            atomicAdd(&b.counters[4], (unsigned long long)G * (unsigned long long)M);
             atomicAdd(&b.counters[6], (unsigned long long)G * (unsigned long long)M);
             atomicAdd(&b.counters[10], (unsigned long long)G);
         }
@@ -2004,7 +2005,6 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
         double* me = b.map_ext[cur ^ 1] + 12 * wrow;
         for (int q = 0; q < 12; ++q) me[q] = fixed ? 0.0 : b.ext[12 * p + q];
         if (cut) atomicAdd(&b.counters[0], 1ull);
-        atomicAdd(&b.counters[5], (unsigned long long)n);
         atomicAdd(&b.counters[7], (unsigned long long)n);
         atomicAdd(&b.counters[11], (unsigned long long)n_out);
         atomicMax(&b.counters[13], (unsigned long long)n_all_surv);
@@ -2110,20 +2110,15 @@ __global__ void __launch_bounds__(kFusedThreads, sizeof(T) == 4 ? 3 : 2)
 }
 
 // The launch before a single filter's fused update: this frame's measurements into the
-// T layout (u, v, d), the per-update counters and the work counter to 0.
+// T layout (u, v, d), the work counter to 0.
 template <typename T, int K>
-__global__ void k_stage_frame(T* z, const double* zu, const double* zv, const double* zd, int M,
-                              unsigned long long* counters, int* work) {
+__global__ void k_stage_frame(T* z, const double* zu, const double* zv, const double* zd, int M, int* work) {
     for (int m = threadIdx.x; m < M; m += blockDim.x) {
         z[m * 3 + 0] = (T)zu[m];
         z[m * 3 + 1] = (T)zv[m];
         z[m * 3 + 2] = (K == 3 && zd) ? (T)zd[m] : T(0);
     }
-    if (threadIdx.x == 0) {
-        counters[4] = 0;
-        counters[5] = 0;
-        *work = 0;
-    }
+    if (threadIdx.x == 0) *work = 0;
 }
 
 // ---------------------------------------------------------------- parent weights
@@ -2148,10 +2143,19 @@ __device__ double block_reduce_max(double v, double* s_tmp) {
     return r;
 }
 
-// log-domain form of .cu:1845-1875: lw += loglik, normalise; N_eff of the result
-__device__ __forceinline__ void weights_body(int N, double* lw, const double* loglik, int apply, double* scal,
-                                             unsigned long long* counters) {
-    if (threadIdx.x == 0 && counters) counters[2] += 1;   // frames updated
+// log-domain form of .cu:1845-1875: lw += loglik, normalise; N_eff of the result.  The
+// update's last launch: also its counters, [4] and [5] what [6] and [7] grew by.  cum (may be
+// null) receives the normalised weights.  Any block width from N up to 1024 gives the same
+// sums (the warps without a parent add zeros).
+__device__ __forceinline__ double weights_body(int N, double* lw, const double* loglik, int apply, double* scal,
+                                               unsigned long long* counters, unsigned long long* snap, double* cum) {
+    if (threadIdx.x == 0) {
+        counters[2] += 1;   // frames updated
+        for (int i = 0; i < 2; ++i) {
+            counters[4 + i] = counters[6 + i] - snap[i];
+            snap[i] = counters[6 + i];
+        }
+    }
     __shared__ double s_tmp[32];
     double mx = -INFINITY;
     for (int p = threadIdx.x; p < N; p += blockDim.x) {
@@ -2169,22 +2173,19 @@ __device__ __forceinline__ void weights_body(int N, double* lw, const double* lo
         double v = lw[p] - ls;
         lw[p] = v;
         double w = exp(v);
+        if (cum) cum[p] = w;
         ss += w * w;
     }
     ss = block_reduce_sum(ss, s_tmp);
-    if (threadIdx.x == 0) scal[0] = 1.0 / (N * ss);   // computeNeff, .cu:2641-2649
+    const double neff = 1.0 / (N * ss);   // computeNeff, .cu:2641-2649
+    if (threadIdx.x == 0) scal[0] = neff;
+    return neff;
 }
-
-__global__ void __launch_bounds__(1024) k_weights(int N, double* lw, const double* loglik, int apply, double* scal,
-                                                  unsigned long long* counters) {
-    weights_body(N, lw, loglik, apply, scal, counters);
-}
+inline int weights_threads(int N) { return N >= 1024 ? 1024 : (N + 31) / 32 * 32; }
 
 template <typename T>
-__global__ void __launch_bounds__(1024) k_weights_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas) {
-    const int f = blockIdx.x;
-    const Bufs<T>& b = tab.b[f];
-    weights_body(tab.prm[f].N, b.lw, b.loglik, fas[f].fixed ? 0 : 1, b.scal, b.counters);
+__global__ void __launch_bounds__(1024) k_weights(__grid_constant__ const Bufs<T> b, int N, int apply) {
+    weights_body(N, b.lw, b.loglik, apply, b.scal, b.counters, b.snap, nullptr);
 }
 
 // ---------------------------------------------------------------- (e) resample
@@ -2224,24 +2225,29 @@ __device__ void block_scan_inclusive(double* data, int N, double* s_tmp) {
 }
 
 // gather_ext = false: the parent states are left for k_gather_parents / k_copy_parents
-// (the single filter's path: the 96-byte rows are moved by the whole GPU, not one block)
+// (a filter of more than kGatherParents parents: its 96-byte rows are moved by the whole GPU,
+// not by one block; 43 -> 23 us at 4096, while two more launches cost what one block takes
+// for 1024).  neff >= 0: the weights are in cum already and this is their N_eff.
+constexpr int kGatherParents = 1024;
 __device__ __forceinline__ void resample_body(const Params& prm, double* lw, double* ext, double* ext_tmp, int* src,
                                               int* src_tmp, double* cum, double* scal, int* flags, int* idx_out,
                                               uint32_t frame, int force, double r0_override,
-                                              unsigned long long* counters, bool gather_ext = true) {
+                                              unsigned long long* counters, bool gather_ext = true, double neff = -1.0) {
     __shared__ double s_tmp[32];
     __shared__ double s_r0;
     __shared__ int s_amax;
     const int N = prm.N;
-    double ss = 0;
-    for (int p = threadIdx.x; p < N; p += blockDim.x) {
-        double w = exp(lw[p]);
-        cum[p] = w;
-        ss += w * w;
+    if (!(neff >= 0.0)) {
+        double ss = 0;
+        for (int p = threadIdx.x; p < N; p += blockDim.x) {
+            double w = exp(lw[p]);
+            cum[p] = w;
+            ss += w * w;
+        }
+        ss = block_reduce_sum(ss, s_tmp);
+        neff = 1.0 / (N * ss);   // computeNeff, .cu:2641-2649
+        if (threadIdx.x == 0) scal[0] = neff;
     }
-    ss = block_reduce_sum(ss, s_tmp);
-    const double neff = 1.0 / (N * ss);   // computeNeff, .cu:2641-2649
-    if (threadIdx.x == 0) scal[0] = neff;
     if (!force && !(neff < prm.min_neff)) {   // .cu:2656-2657
         if (threadIdx.x == 0) flags[0] = 0;
         return;
@@ -2342,17 +2348,30 @@ __global__ void k_copy_parents(const int* flags, const double* ext_tmp, double* 
     ext[e] = ext_tmp[e];
 }
 
+// A step's two last stages in one launch: the weights' N_eff and linear weights are at hand
+// when the resampling starts (256 parents: 10.7 + 14.4 us in two launches and two gathers)
 template <typename T>
-__global__ void __launch_bounds__(1024) k_resample_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas) {
-    const int f = blockIdx.x;
-    const Bufs<T>& b = tab.b[f];
-    resample_body(tab.prm[f], b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal, b.flags, b.resample_idx,
-                  fas[f].frame, 0, -1.0, b.counters);
+__global__ void __launch_bounds__(1024)
+    k_weights_resample(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int apply, uint32_t frame) {
+    const double neff = weights_body(prm.N, b.lw, b.loglik, apply, b.scal, b.counters, b.snap, b.cum);
+    __syncthreads();
+    resample_body(prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal, b.flags, b.resample_idx, frame, 0, -1.0,
+                  b.counters, prm.N <= kGatherParents, neff);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas) {
+    const Bufs<T>& b = tab.b[blockIdx.x];
+    const Params& prm = tab.prm[blockIdx.x];
+    const FrameArgs& fa = fas[blockIdx.x];
+    const double neff = weights_body(prm.N, b.lw, b.loglik, fa.fixed ? 0 : 1, b.scal, b.counters, b.snap, b.cum);
+    __syncthreads();
+    resample_body(prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal, b.flags, b.resample_idx, fa.frame, 0, -1.0,
+                  b.counters, true, neff);
 }
 
 // map entry: (filter, first parent of a 256-parent block).  The first block of each
-// filter also resets its per-update counters and converts its frame's measurements
-// into the T layout (u, v, d) for the fused update; block 0 resets the group's work
+// filter also converts its frame's measurements into the T layout (u, v, d) for the fused update; block 0 resets the group's work
 // counter (may be null).
 template <typename T>
 __global__ void k_predict_parents_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map,
@@ -2361,10 +2380,6 @@ __global__ void k_predict_parents_batch(const __grid_constant__ SlotTable<T> tab
     const Bufs<T>& b = tab.b[fp.x];
     const FrameArgs& fa = fas[fp.x];
     if (fp.y == 0) {
-        if (threadIdx.x == 0) {   // counters of "the last update" start at 0
-            b.counters[4] = 0;
-            b.counters[5] = 0;
-        }
         if (fa.zu != nullptr) {
             const int K = tab.prm[fp.x].K;
             for (int m = threadIdx.x; m < fa.M; m += blockDim.x) {
@@ -2379,76 +2394,110 @@ __global__ void k_predict_parents_batch(const __grid_constant__ SlotTable<T> tab
 }
 
 // ---------------------------------------------------------------- cloud materialisation
-// Write the Euclidean cloud of every entry of the maps into dst (rows p*Gcap + j),
-// optionally applying a pending feature prediction (the path of predict() called
-// twice without an update, and the cloud dump of scphd_get_map_clouds).
+// The Euclidean cloud of every entry of the maps into dst (rows p*Gcap + j), with a pending
+// feature prediction applied (predict() called twice without an update).
+
+// sample s of entry j of the map that parent p reads (row `row`): the particle X, with a pending
+// prediction applied; returns its weight
+template <typename T>
+__device__ __forceinline__ T map_sample(const Params& prm, const Bufs<T>& b, int cur, int row, int p, int j, int s,
+                                        const Pose<T>& pose_src, int has_pred, double dt, uint32_t pred_frame,
+                                        uint32_t sample_frame, T (&X)[6]) {
+    const auto& m = ModelOf<T>::get(prm);   // the constants the cloud fit regenerates samples with
+    const int P = prm.P, Ps = prm.Ps;
+    const size_t erow = (size_t)row * prm.Gcap + j;
+    const T* ent = b.map[cur] + erow * kRow;
+    const T* L = ent + 7;   // merged component: Cholesky factor stored in the map row
+    const int ref = b.map_ref[cur][erow];
+    T om;
+    if (ref < 0) {
+        uint32_t w0[4], w1[4];
+        const uint32_t key_i = (uint32_t)(-1 - ref);
+        philox((uint32_t)s, key_i, (uint32_t)row, ctr_word3(sample_frame, ST_SAMPLE, 0), prm.key0, prm.key1, w0);
+        philox((uint32_t)s, key_i, (uint32_t)row, ctr_word3(sample_frame, ST_SAMPLE, 1), prm.key0, prm.key1, w1);
+        T z[6];
+        Pair<T>::two(w0[0], w0[1], z[0], z[1]);
+        Pair<T>::two(w0[2], w0[3], z[2], z[3]);
+        Pair<T>::two(w1[0], w1[1], z[4], z[5]);
+        T y[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            T v = 0;
+#pragma unroll
+            for (int c = 0; c <= a; ++c) v += L[tri(a, c)] * z[c];
+            y[a] = v + ent[1 + a];
+        }
+        invert(y, pose_src, m, X);
+        om = T(1) / T(P);
+    } else {
+        const T* sc = b.cloud[cur] + (size_t)ref * 7 * Ps;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) X[a] = sc[a * Ps + s];
+        om = sc[6 * Ps + s];
+    }
+    if (has_pred) {
+        uint32_t w[4];
+        philox((uint32_t)s, (uint32_t)j, (uint32_t)p, ctr_word3(pred_frame, ST_FEAT, 0), prm.key0, prm.key1, w);
+        T z[4];
+        Pair<T>::two(w[0], w[1], z[0], z[1]);
+        Pair<T>::two(w[2], w[3], z[2], z[3]);
+        const T dtT = (T)dt, half_dt2 = T(0.5) * (T)dt * (T)dt;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            T a = ModelOf<T>::feat_std(prm, q) * z[q];
+            X[q] = X[q] + X[q + 3] * dtT + a * half_dt2;
+            X[q + 3] = X[q + 3] + a * dtT;
+        }
+    }
+    return om;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_materialize(Params prm, Bufs<T> b, int cur, T* dst, T* dst_map,
                                                      int* dst_ref, int* dst_n, int has_pred, double dt,
-                                                     uint32_t pred_frame, uint32_t sample_frame, int only_p) {
-    const int p = only_p >= 0 ? only_p : blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+                                                     uint32_t pred_frame, uint32_t sample_frame) {
+    const int p = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = b.src[p];
     const int G = min(b.map_n[cur][row], prm.Gcap);
     __shared__ Pose<T> pose_src;
     if (threadIdx.x == 0) pose_src = make_pose<T>(b.map_ext[cur] + 12 * row);
     __syncthreads();
-    const auto& m = ModelOf<T>::get(prm);   // the constants the cloud fit regenerates samples with
     const int P = prm.P, Ps = prm.Ps;
     for (int j = warp; j < G; j += blockDim.x >> 5) {
-        const size_t erow = (size_t)row * prm.Gcap + j;
-        const T* ent = b.map[cur] + erow * kRow;
-        const int ref = b.map_ref[cur][erow];
-        T W = ent[0];
-        const T* L = ent + 7;   // merged component: Cholesky factor stored in the map row
-        T* cl = dst + ((size_t)(only_p >= 0 ? 0 : p) * prm.Gcap + j) * 7 * Ps;
+        T* cl = dst + ((size_t)p * prm.Gcap + j) * 7 * Ps;
         for (int s = lane; s < P; s += 32) {
-            T X[6], om;
-            if (ref < 0) {
-                uint32_t w0[4], w1[4];
-                const uint32_t key_i = (uint32_t)(-1 - ref);
-                philox((uint32_t)s, key_i, (uint32_t)row, ctr_word3(sample_frame, ST_SAMPLE, 0), prm.key0, prm.key1, w0);
-                philox((uint32_t)s, key_i, (uint32_t)row, ctr_word3(sample_frame, ST_SAMPLE, 1), prm.key0, prm.key1, w1);
-                T z[6];
-                Pair<T>::two(w0[0], w0[1], z[0], z[1]);
-                Pair<T>::two(w0[2], w0[3], z[2], z[3]);
-                Pair<T>::two(w1[0], w1[1], z[4], z[5]);
-                T y[6];
-                for (int a = 0; a < 6; ++a) {
-                    T v = 0;
-                    for (int c = 0; c <= a; ++c) v += L[tri(a, c)] * z[c];
-                    y[a] = v + ent[1 + a];
-                }
-                invert(y, pose_src, m, X);
-                om = T(1) / T(P);
-            } else {
-                const T* sc = b.cloud[cur] + (size_t)ref * 7 * Ps;
-                for (int a = 0; a < 6; ++a) X[a] = sc[a * Ps + s];
-                om = sc[6 * Ps + s];
-            }
-            if (has_pred) {
-                uint32_t w[4];
-                philox((uint32_t)s, (uint32_t)j, (uint32_t)p, ctr_word3(pred_frame, ST_FEAT, 0), prm.key0, prm.key1, w);
-                T z[4];
-                Pair<T>::two(w[0], w[1], z[0], z[1]);
-                Pair<T>::two(w[2], w[3], z[2], z[3]);
-                const T dtT = (T)dt, half_dt2 = T(0.5) * (T)dt * (T)dt;
-                for (int q = 0; q < 3; ++q) {
-                    T a = ModelOf<T>::feat_std(prm, q) * z[q];
-                    X[q] = X[q] + X[q + 3] * dtT + a * half_dt2;
-                    X[q + 3] = X[q + 3] + a * dtT;
-                }
-            }
+            T X[6];
+            const T om = map_sample(prm, b, cur, row, p, j, s, pose_src, has_pred, dt, pred_frame, sample_frame, X);
             for (int a = 0; a < 6; ++a) cl[a * Ps + s] = X[a];
             cl[6 * Ps + s] = om;
         }
-        if (dst_map != nullptr && lane == 0) {
+        if (lane == 0) {
+            const T W = b.map[cur][((size_t)row * prm.Gcap + j) * kRow];
             T* o = dst_map + ((size_t)p * prm.Gcap + j) * kRow;
             o[0] = has_pred ? W * (T)prm.ps : W;
             dst_ref[(size_t)p * prm.Gcap + j] = p * prm.Gcap + j;
         }
     }
-    if (dst_n != nullptr && threadIdx.x == 0) dst_n[p] = G;
+    if (threadIdx.x == 0) dst_n[p] = G;
+}
+
+// The cloud of one parent's map for the host: a thread per sample over the whole GPU (one block
+// of eight warps took 200 us for 103 Gaussians of 100 FP64 samples), written in FP64 in the
+// order the caller gets it: xyz G x 6 x P, om G x P.
+template <typename T>
+__global__ void __launch_bounds__(128) k_map_cloud(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int cur,
+                                                   double* xyz, double* om, int G, int has_pred, double dt,
+                                                   uint32_t pred_frame, uint32_t sample_frame, int p) {
+    const int row = b.src[p];
+    __shared__ Pose<T> pose_src;
+    if (threadIdx.x == 0) pose_src = make_pose<T>(b.map_ext[cur] + 12 * row);
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = i / prm.P, s = i - j * prm.P;
+    if (j >= G) return;
+    T X[6];
+    om[(size_t)j * prm.P + s] = (double)map_sample(prm, b, cur, row, p, j, s, pose_src, has_pred, dt, pred_frame, sample_frame, X);
+#pragma unroll
+    for (int a = 0; a < 6; ++a) xyz[((size_t)j * 6 + a) * prm.P + s] = (double)X[a];
 }
 
 // ---------------------------------------------------------------- stand-alone merge
