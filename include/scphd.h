@@ -289,8 +289,9 @@ scphd_status scphd_device_bytes(const scphd_config* cfg, int64_t* bytes);
  * precision and meas_dim; they may differ in size.  While in a batch, the filters
  * issue all their work on the batch's stream (their own stream is restored by
  * scphd_batch_destroy), so single-filter calls stay ordered with batched steps.  With
- * use_graph != 0 the first step captures the step into a CUDA graph and later steps
- * replay it.  A batched step gives each filter the same result as predict + update +
+ * use_graph != 0 the step is captured into a CUDA graph once its launch shapes are tuned
+ * (on maps that have grown: after 16 frames of every member and six timed steps), and
+ * later steps replay it.  A batched step gives each filter the same result as predict + update +
  * resample on that filter alone.  This batching has no counterpart in the reference
  * (which runs one filter per process). */
 typedef struct scphd_frame {
@@ -323,8 +324,9 @@ void* scphd_batch_stream(scphd_batch* b);
 scphd_status scphd_batch_set_fused(scphd_batch* b, int32_t mode);
 scphd_status scphd_batch_get_fused(scphd_batch* b, int32_t* fused);
 /* The batch's cloud-fit tiling, as scphd_set_fit_split / scphd_get_fit_split (one
- * split for all member filters, tuned on the batch's first six steps before its graph
- * is captured; set it before the capture). */
+ * split for all member filters, tuned with the merge's block width on six steps once
+ * every member has seen 16 frames, before the batch's graph is captured; set it before
+ * the capture). */
 scphd_status scphd_batch_set_fit_split(scphd_batch* b, int32_t blocks_per_parent);
 scphd_status scphd_batch_get_fit_split(scphd_batch* b, int32_t* blocks_per_parent, int32_t* tuned);
 

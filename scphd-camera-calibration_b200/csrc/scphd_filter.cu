@@ -1329,7 +1329,7 @@ template <typename T> struct Batch final : scphd_batch {
         int4* map_lik = nullptr;    int n_lik = 0;
         int* work = nullptr;            // the fused update's work counter
         bool fit_p = false;             // every member has kFitP samples per feature
-        int merge_over = 0;             // blocks per filter of the second merge launch (0: none needed)
+        int merge_over[3] = {0, 0, 0};  // blocks per filter of the second merge launch, by width (0: none needed)
     };
     int K = 3;
     bool use_graph = false;
@@ -1346,30 +1346,34 @@ template <typename T> struct Batch final : scphd_batch {
     std::vector<size_t> stage_off;
     size_t stage_total = 0;
     size_t merge_smem = 0;       // the members' full survivor capacities
-    size_t merge_first_smem = 0; // the first launch's (Params::Ssm)
+    size_t merge_first_smem[3] = {0, 0, 0};   // the first launch's (Params::Ssm), by width
     size_t merge_need = 0;       // the limit's (merge_limit_bytes)
     size_t fit_smem = 0;
     size_t lik_smem = 0;
     int lik_block = 32;
-    // the update path: the stage kernels with 256 or 128 threads per merge block, tuned
-    // on the first 4 steps before a graph is captured (twice each; results do not depend
-    // on it), or the fused kernel when requested (scphd_batch_set_fused)
-    static constexpr int kPaths = 2;
-    int path = 0;              // 0, 1: stage kernels (merge 256 / 128 threads)
+    // the update path: the stage kernels with 256, 128 or 64 threads per merge block, or the
+    // fused kernel when requested (scphd_batch_set_fused).  The width is tuned by the merge
+    // launches' own time, twice each, with the cloud fit's split below, on the first six steps
+    // whose members have all seen kTuneAfter frames (their maps have grown: at 64 filters of 256
+    // parents the first frames' maps chose 256 threads, 64 are 1.2 times as fast); the graph is
+    // captured after them.  Results do not depend on either.
+    static constexpr int kPaths = 3, kTuneAfter = 16;
+    const int merge_widths[kPaths] = {kMergeThreads, 128, 64};
+    int path = 0;
+    bool ripe = false;         // every member has seen kTuneAfter frames
     int fused_mode = 0;        // 1: the fused kernel instead
     size_t fused_smem = 0;
     int fused_grid = 0;        // 0: the fused kernel is unavailable
     bool tuning = true;
     bool capturing = false;
     int tune_trials = 0, tune_pending = -1;
-    double tune_ms[kPaths] = {0, 0};
-    int path_now() const {     // the path of the step being enqueued (2: fused)
-        if (fused_mode == 1 && fused_grid > 0) return 2;
-        return (tuning && !capturing) ? tune_trials % kPaths : path;
+    double tune_ms[kPaths] = {0, 0, 0};
+    int path_now() const {     // the path of the step being enqueued (kPaths: fused)
+        if (fused_mode == 1 && fused_grid > 0) return kPaths;
+        return (tuning && ripe && !capturing) ? tune_trials % kPaths : path;
     }
     cudaEvent_t tune_ev[2] = {nullptr, nullptr};
-    // blocks per parent of the cloud fit, tuned on the first six steps (1, 2, 4, twice
-    // each) by the cloud-fit launches' own time, before the graph is captured
+    // blocks per parent of the cloud fit (1, 2, 4), tuned by the cloud-fit launches' own time
     static constexpr int kFitSplits = 3;
     const int fit_splits[kFitSplits] = {1, 2, 4};
     bool fit_tuning = true;
@@ -1438,10 +1442,13 @@ template <typename T> struct Batch final : scphd_batch {
                 stage_total += 3 * (size_t)pr.Mcap;
                 merge_need = std::max(merge_need, merge_limit_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
                 merge_smem = std::max(merge_smem, merge_shared_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
-                const int S = merge_launch_cap<T>(pr.Scap, pr.Gcap, kMergeThreads, kMergeBlocks<T>);
-                g.tab->prm[i].Ssm = S;
-                merge_first_smem = std::max(merge_first_smem, merge_shared_bytes<T>(S, pr.Gcap, kMergeThreads / 32));
-                if (S < pr.Scap) g.merge_over = std::max(g.merge_over, std::min(pr.N, 16));
+                for (int w = 0; w < kPaths; ++w) {
+                    const int threads = merge_widths[w];
+                    const int S = merge_launch_cap<T>(pr.Scap, pr.Gcap, threads, kMergeBlocks<T> * (kMergeThreads / threads));
+                    g.tab->prm[i].Ssm[w] = S;
+                    merge_first_smem[w] = std::max(merge_first_smem[w], merge_shared_bytes<T>(S, pr.Gcap, threads / 32));
+                    if (S < pr.Scap) g.merge_over[w] = std::max(g.merge_over[w], std::min(pr.N, 16));
+                }
                 fit_smem = std::max(fit_smem, fit_kernel_smem_bytes<T>(pr.P));
                 fused_smem = std::max(fused_smem, fused_smem_bytes<T>(pr.P, pr.Gcap, pr.Scap));
                 lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block));
@@ -1517,21 +1524,20 @@ template <typename T> struct Batch final : scphd_batch {
     // kernels of one frame, stage by stage over the groups
     template <int KK> scphd_status launch_all() {
         const int pth = path_now();
-        const bool timed = tuning && !capturing && pth < kPaths;
-        if (timed) CUDA_TRY(cudaEventRecord(tune_ev[0], stream));
+        const bool timed = tuning && ripe && !capturing && pth < kPaths;
         for (const Group& g : groups) {
             k_predict_parents_batch<T><<<g.n_pred, 256, 0, stream>>>(*g.tab, d_fa + g.first, g.map_pred,
-                                                                     pth == 2 ? g.work : nullptr);
+                                                                     pth == kPaths ? g.work : nullptr);
             LAUNCHED();
         }
-        if (pth == 2) {
+        if (pth == kPaths) {
             for (const Group& g : groups) {
                 k_fused_batch<T, KK><<<std::min(g.n_parent, fused_grid), kFusedThreads, fused_smem, stream>>>(
                     *g.tab, d_fa + g.first, g.map_parent, g.n_parent, g.work);
                 LAUNCHED();
             }
         } else {
-            const bool fit_timed = fit_tuning && !capturing;
+            const bool fit_timed = fit_tuning && ripe && !capturing;
             const int fsi = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fsi];
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             for (const Group& g : groups) {
@@ -1556,33 +1562,34 @@ template <typename T> struct Batch final : scphd_batch {
                 k_likelihood_batch<T, KK><<<g.n_lik, lik_block, lik_smem, stream>>>(*g.tab, d_fa + g.first, g.map_lik);
                 LAUNCHED();
             }
-            const int mt = pth == 1 ? 128 : kMergeThreads;
+            if (timed) CUDA_TRY(cudaEventRecord(tune_ev[0], stream));
             for (const Group& g : groups) {
-                k_merge_batch<T, KK><<<g.n_parent, mt, merge_first_smem, stream>>>(*g.tab, d_fa + g.first, g.map_parent,
-                                                                                   g.count, 0);
+                k_merge_batch<T, KK><<<g.n_parent, merge_widths[pth], merge_first_smem[pth], stream>>>(
+                    *g.tab, d_fa + g.first, g.map_parent, g.count, pth, 0);
                 LAUNCHED();
             }
             for (const Group& g : groups) {
-                if (!g.merge_over) continue;
-                k_merge_batch<T, KK><<<g.count * g.merge_over, kMergeThreads, merge_smem, stream>>>(*g.tab, d_fa + g.first,
-                                                                                                   g.map_parent, g.count, 1);
+                if (!g.merge_over[pth]) continue;
+                k_merge_batch<T, KK><<<g.count * g.merge_over[pth], kMergeThreads, merge_smem, stream>>>(
+                    *g.tab, d_fa + g.first, g.map_parent, g.count, pth, 1);
                 LAUNCHED();
+            }
+            if (timed) {
+                CUDA_TRY(cudaEventRecord(tune_ev[1], stream));
+                tune_pending = pth;
             }
         }
         for (const Group& g : groups) {
             k_weights_resample_batch<T><<<g.count, 1024, 0, stream>>>(*g.tab, d_fa + g.first);
             LAUNCHED();
         }
-        if (timed) {
-            CUDA_TRY(cudaEventRecord(tune_ev[1], stream));
-            tune_pending = tune_trials % kPaths;
-        }
         return SCPHD_OK;
     }
 
     int launches_per_frame() const {
         int n = 0;
-        for (const Group& g : groups) n += path_now() == 2 ? 3 : 6 + (g.merge_over > 0);
+        const int pth = path_now();
+        for (const Group& g : groups) n += pth == kPaths ? 3 : 6 + (g.merge_over[pth] > 0);
         return n;
     }
 
@@ -1595,7 +1602,7 @@ template <typename T> struct Batch final : scphd_batch {
         if (mode == 1) tuning = fit_tuning = false;   // the stage kernels' shapes are not needed
         return SCPHD_OK;
     }
-    int fused_path() const override { return path_now() == 2 ? 1 : 0; }
+    int fused_path() const override { return path_now() == kPaths ? 1 : 0; }
     scphd_status set_fit_split(int blocks_per_parent) override {
         if (captured) return fail(SCPHD_ERR_INVALID, "the batch's step graph is already captured");
         for (int k = 0; k < kFitSplits; ++k)
@@ -1633,7 +1640,8 @@ template <typename T> struct Batch final : scphd_batch {
         tune_pending = -1;
         if (++tune_trials >= 2 * kPaths) {
             tuning = false;
-            path = tune_ms[1] < tune_ms[0] ? 1 : 0;
+            for (int k = 1; k < kPaths; ++k)
+                if (tune_ms[k] < tune_ms[path]) path = k;
         }
         return SCPHD_OK;
     }
@@ -1703,6 +1711,10 @@ template <typename T> struct Batch final : scphd_batch {
         {
             const scphd_status ts = tune_collect();
             if (ts != SCPHD_OK) return ts;
+        }
+        if (!ripe) {
+            ripe = true;
+            for (int f = 0; f < F; ++f) ripe = ripe && filt(f)->frame > kTuneAfter;
         }
         {
             const scphd_status cs = copy_in();

@@ -26,7 +26,7 @@ namespace scphd {
 
 struct Params {
     int N, P, Ps, Gcap, Mcap, Scap, K;
-    int Ssm;         // survivor capacity of a batch's first merge launch (merge_launch_cap)
+    int Ssm[3];      // survivor capacity of a batch's first merge launch of 256, 128, 64 threads (merge_launch_cap)
     Model model;
     ModelF model_f;   // model's transform constants in FP32
     double kappa, ps, min_weight, min_sep, min_neff;
@@ -2029,14 +2029,15 @@ __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
 // filter, its listed parents are dealt out over that filter's blocks
 template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
-    k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int over) {
+    k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int width,
+                  int over) {
     const int2 fp = over ? make_int2(blockIdx.x % count, blockIdx.x / count) : map[blockIdx.x];
     const Params& prm = tab.prm[fp.x];
     const Bufs<T>& b = tab.b[fp.x];
     const FrameArgs fa = fas[fp.x];
     const int n = over ? min(b.flags[3], prm.N) : fp.y + 1, step = over ? gridDim.x / count : 1;
     for (int i = fp.y; i < n; i += step) {
-        merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, over ? b.src_tmp[i] : i, over ? prm.Scap : prm.Ssm);
+        merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, over ? b.src_tmp[i] : i, over ? prm.Scap : prm.Ssm[width]);
         __syncthreads();
     }
 }
