@@ -186,8 +186,10 @@ scphd_status scphd_get_counters(scphd_filter* f, int64_t counters[16]);
  * per merge block (256 or 128) and the likelihood's blocks (1: one block over all of a
  * parent's measurements, 0: 128-thread blocks).  Each of the four combinations runs
  * twice, timed with events (those updates wait for the previous one), and the fastest is
- * kept.  Results do not depend on the shape.  enable = 0 stops tuning and keeps
- * (256, 1); *tuned = 1 once a choice is made.  No reference counterpart. */
+ * kept.  The merge's width is timed again on grown maps, twice each on the updates with
+ * measurements after the first 22 (64 threads among them for a filter of many parents).
+ * Results do not depend on the shape.  enable = 0 stops tuning and keeps (256, 1);
+ * *tuned = 1 once the first choice is made.  No reference counterpart. */
 scphd_status scphd_set_autotune(scphd_filter* f, int32_t enable);
 scphd_status scphd_get_launch_shapes(scphd_filter* f, int32_t* merge_threads, int32_t* likelihood_full,
                                      int32_t* tuned);

@@ -124,6 +124,19 @@ struct scphd_filter {
     int fit_trials = 0, fit_pending = -1, fit_chosen = 0;
     double fit_ms[kFitSplits] = {0, 0, 0};
     cudaEvent_t fit_ev[2] = {nullptr, nullptr};
+    // Threads per merge block on grown maps: the first updates' choice (shapes) rests on maps of
+    // a few components, so the widths are timed again, by the merge launches' own time, twice
+    // each on the updates after the cloud fit's, and 64 threads with them for a filter whose
+    // blocks of 128 are not all resident at once (4096 parents x 256 Gaussians: 256 threads 0.50,
+    // 128 0.39, 64 0.72 ms; 1024 x 128: 90, 90, 76 us).  The choice is -1 until then.
+    static constexpr int kMergeWidths = 3, kMergeTuneAfter = kFitTuneAfter + 2 * kFitSplits;
+    const int merge_widths[kMergeWidths] = {kMergeThreads, 128, 64};
+    int merge_candidates = 2;
+    bool merge_tuning = true;
+    int merge_trials = 0, merge_pending = -1, merge_chosen = -1;
+    double merge_ms[kMergeWidths] = {0, 0, 0};
+    cudaEvent_t merge_ev[2] = {nullptr, nullptr};
+    int merge_width() const { return merge_chosen >= 0 ? merge_chosen : (shapes[chosen].merge_threads == kMergeThreads ? 0 : 1); }
     // whether the next update takes the fused path (profiling times the stage kernels
     // one by one)
     bool fused_next() const { return fused_mode == 1 && !profiling && fused_grid > 0; }
@@ -144,6 +157,19 @@ struct scphd_filter {
                 fit_tuning = false;
                 for (int k = 1; k < kFitSplits; ++k)
                     if (fit_ms[k] < fit_ms[fit_chosen]) fit_chosen = k;
+            }
+        }
+        if (merge_pending >= 0) {
+            CUDA_TRY(cudaEventSynchronize(merge_ev[1]));
+            float ms = 0;
+            CUDA_TRY(cudaEventElapsedTime(&ms, merge_ev[0], merge_ev[1]));
+            merge_ms[merge_pending] += ms;
+            merge_pending = -1;
+            if (++merge_trials >= 2 * merge_candidates) {
+                merge_tuning = false;
+                merge_chosen = 0;
+                for (int k = 1; k < merge_candidates; ++k)
+                    if (merge_ms[k] < merge_ms[merge_chosen]) merge_chosen = k;
             }
         }
         if (tune_pending < 0) return SCPHD_OK;
@@ -206,6 +232,8 @@ struct scphd_filter {
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : fit_ev)
             if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : merge_ev)
+            if (e) cudaEventDestroy(e);
     }
     virtual scphd_status init() = 0;
     virtual scphd_status predict(double dt) = 0;
@@ -244,7 +272,7 @@ public:
     double* dump = nullptr;   // Gcap x 7 x P: a parent's cloud for the host
     size_t merge_smem = 0;       // the full survivor capacity's
     int merge_over_grid = 0;     // blocks of the second merge launch
-    struct MergeLaunch { int S = 0; size_t smem = 0; } merge_at[2];   // first launch: kMergeThreads, 128 threads
+    struct MergeLaunch { int S = 0; size_t smem = 0; } merge_at[kMergeWidths];   // first launch, by width
     size_t fit_smem = 0;
 
     ~Filter() override {
@@ -300,6 +328,8 @@ public:
         CUDA_TRY(cudaEventCreate(&tune_ev[1]));
         CUDA_TRY(cudaEventCreate(&fit_ev[0]));
         CUDA_TRY(cudaEventCreate(&fit_ev[1]));
+        CUDA_TRY(cudaEventCreate(&merge_ev[0]));
+        CUDA_TRY(cudaEventCreate(&merge_ev[1]));
         CUDA_TRY(cudaEventCreateWithFlags(&stage_ev, cudaEventDisableTiming));
         CUDA_TRY(cudaMallocHost(&h_stage, sizeof(double) * 3 * prm.Mcap));
         Arena probe;
@@ -348,8 +378,9 @@ public:
             CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, merge_fn, kMergeThreads, merge_smem));
             merge_over_grid = std::min(prm.N, nsm * occ);
             // a filter whose parents are all resident at the full capacity takes one launch
-            for (int k = 0; k < 2; ++k) {
-                const int threads = k == 0 ? kMergeThreads : 128, blocks = kMergeBlocks<T> * (kMergeThreads / threads);
+            merge_candidates = prm.N > nsm * kMergeBlocks<T> * 2 ? 3 : 2;
+            for (int k = 0; k < kMergeWidths; ++k) {
+                const int threads = merge_widths[k], blocks = kMergeBlocks<T> * (kMergeThreads / threads);
                 merge_at[k].S = prm.N <= merge_over_grid ? prm.Scap : merge_launch_cap<T>(prm.Scap, prm.Gcap, threads, blocks);
                 merge_at[k].smem = merge_shared_bytes<T>(merge_at[k].S, prm.Gcap, threads / 32);
             }
@@ -433,6 +464,9 @@ public:
             const double* zs[3] = {M > 0 ? d_stage : nullptr, M > 0 ? d_stage + M : nullptr,
                                    M > 0 ? d_stage + 2 * M : nullptr};
             const bool fit_timed = fit_tuning && M > 0 && fit_seen >= kFitTuneAfter;
+            const bool merge_timed = merge_tuning && !tuning && M > 0 && fit_seen >= kMergeTuneAfter;
+            const int mw = merge_timed ? merge_trials % merge_candidates
+                                       : (merge_chosen >= 0 ? merge_chosen : (sh.merge_threads == kMergeThreads ? 0 : 1));
             if (M > 0) ++fit_seen;
             const int fs = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fs];
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
@@ -463,12 +497,17 @@ public:
                 stage_end(h);
             }
             h = stage_begin(3);
-            const MergeLaunch& ml = merge_at[sh.merge_threads == kMergeThreads ? 0 : 1];
-            k_merge<T, K><<<N, sh.merge_threads, ml.smem, stream>>>(prm, b, cur, M, fixed, ml.S, 0);
+            const MergeLaunch& ml = merge_at[mw];
+            if (merge_timed) CUDA_TRY(cudaEventRecord(merge_ev[0], stream));
+            k_merge<T, K><<<N, merge_widths[mw], ml.smem, stream>>>(prm, b, cur, M, fixed, ml.S, 0);
             LAUNCHED();
             if (ml.S < prm.Scap) {
                 k_merge<T, K><<<merge_over_grid, kMergeThreads, merge_smem, stream>>>(prm, b, cur, M, fixed, prm.Scap, 1);
                 LAUNCHED();
+            }
+            if (merge_timed) {
+                CUDA_TRY(cudaEventRecord(merge_ev[1], stream));
+                merge_pending = mw;
             }
             stage_end(h);
         }
@@ -998,6 +1037,9 @@ scphd_status scphd_set_autotune(scphd_filter* f, int32_t enable) {
         f->fit_tuning = false;
         f->fit_pending = -1;
         f->fit_chosen = 0;
+        f->merge_tuning = false;
+        f->merge_pending = -1;
+        f->merge_chosen = -1;
     }
     return SCPHD_OK;
 }
@@ -1025,7 +1067,7 @@ scphd_status scphd_get_launch_shapes(scphd_filter* f, int32_t* merge_threads, in
                                      int32_t* tuned) {
     if (!f) return fail(SCPHD_ERR_INVALID, "null handle");
     const scphd_filter::Shape& sh = f->shapes[f->chosen];
-    if (merge_threads) *merge_threads = sh.merge_threads;
+    if (merge_threads) *merge_threads = f->merge_widths[f->merge_width()];
     if (likelihood_full) *likelihood_full = sh.lik_full;
     if (tuned) *tuned = f->tuning ? 0 : 1;
     return SCPHD_OK;
