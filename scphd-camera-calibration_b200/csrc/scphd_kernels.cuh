@@ -104,6 +104,17 @@ template <typename T> struct SlotTable {
 // kernel parameters are limited to 32764 bytes: the table plus two pointers must fit
 static_assert(sizeof(SlotTable<double>) + 64 <= 32764, "batch parameter table exceeds the kernel parameter limit");
 
+// First statement of a kernel of a step's chain (scphd_filter.cu, chained): the kernel waits for
+// the end of the one before it; an ordinary launch passes at once.  In a batch the next kernel
+// may take the slots this one's last blocks leave free (64 filters of 256 parents: 2.43 -> 2.36
+// ms per step); a single filter's next kernel starts when this one's blocks have ended, since
+// waiting blocks would keep other filters' kernels from those slots (three filters of 1024
+// parents side by side: 291 us per step, 310 with early blocks, 289 so).
+template <bool kBatch = false> __device__ __forceinline__ void chain_wait() {
+    if (kBatch) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t tie_key(uint32_t r) {
     // argmax order of phdUpdateMergeKernel (src/kernels.cu:704-739) on equal weights:
     // earliest index within a thread's stride, then bit-reversed thread slot.
@@ -154,6 +165,7 @@ __device__ __forceinline__ void predict_parents_body(const Params& prm, double* 
 }
 
 __global__ void k_predict_parents(__grid_constant__ const Params prm, double* ext, double dt, uint32_t frame) {
+    chain_wait();
     predict_parents_body(prm, ext, dt, frame, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -638,6 +650,7 @@ __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
     k_cloud_fit(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int cur, int M, int fixed,
                 int has_pred, double dt, uint32_t pred_frame, uint32_t sample_frame, const double* zu,
                 const double* zv, const double* zd, int split) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_fit[];
     const int p = blockIdx.x / split;
     cloud_fit_any<T, K, PC>(prm, b, cur, M, fixed, has_pred, dt, pred_frame, sample_frame, zu, zv, zd, p,
@@ -647,6 +660,7 @@ __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
 template <typename T, int K, int PC = 0>
 __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
     k_cloud_fit_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int split) {
+    chain_wait<true>();
     extern __shared__ __align__(16) unsigned char dsm_fit[];
     const int q = blockIdx.x / split;
     const int2 fp = map[q];
@@ -745,6 +759,7 @@ __device__ __forceinline__ void prep_body(const Params& prm, const Bufs<T>& b, i
 template <typename T, int K>
 __global__ void __launch_bounds__(kPrepThreads) k_prep(__grid_constant__ const Params prm,
                                                        __grid_constant__ const Bufs<T> b, int cur) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_prep[];
     prep_body<T, K>(prm, b, cur, blockIdx.x, reinterpret_cast<T*>(dsm_prep));
 }
@@ -752,6 +767,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(__grid_constant__ const P
 template <typename T, int K>
 __global__ void __launch_bounds__(kPrepThreads)
     k_prep_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map) {
+    chain_wait<true>();
     extern __shared__ __align__(16) unsigned char dsm_prep[];
     const int2 fp = map[blockIdx.x];
     prep_body<T, K>(tab.prm[fp.x], tab.b[fp.x], fas[fp.x].cur, fp.y, reinterpret_cast<T*>(dsm_prep));
@@ -967,6 +983,7 @@ __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>
 template <typename T, int K>
 __global__ void __launch_bounds__(1024) k_likelihood(__grid_constant__ const Params prm,
                                                      __grid_constant__ const Bufs<T> b, int cur, int M) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_lik[];
     likelihood_body<T, K>(prm, b, cur, M, blockIdx.x, blockIdx.y, reinterpret_cast<T*>(dsm_lik));
 }
@@ -975,6 +992,7 @@ __global__ void __launch_bounds__(1024) k_likelihood(__grid_constant__ const Par
 template <typename T, int K>
 __global__ void __launch_bounds__(1024)
     k_likelihood_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int4* map) {
+    chain_wait<true>();
     extern __shared__ __align__(16) unsigned char dsm_lik[];
     const int4 e = map[blockIdx.x];
     const int M = fas[e.x].M;
@@ -1371,12 +1389,17 @@ __device__ inline void carve_merge_shared(unsigned char* smem, int S, int G, T*&
 // a second one at the full capacity (4 us when the list is empty): 4.6 -> 2.8 ms and, in
 // FP64, 1.96 -> 1.32 ms at those sizes.  From two blocks to three the gain is 5 %, less at
 // few parents: that is left to the layout (FP32 at 968 survivors: three fit).
+// A launch holds 1.5 times the map capacity at least, on fewer blocks if need be: a grown
+// map's parents have 1 to 1.4 times its components as survivors.
 template <typename T> inline int merge_launch_cap(int Scap, int G, int threads, int blocks) {
     auto room = [](int n) { return (size_t)228 * 1024 / n - 1024 - 3584; };   // less what a block reserves, and static
     if (merge_shared_bytes<T>(Scap, G, threads / 32) <= room(blocks / 2 + 1)) return Scap;
-    int S = 0;
-    while (S + 32 <= Scap && merge_shared_bytes<T>(S + 32, G, threads / 32) <= room(blocks)) S += 32;
-    return S >= G ? S : Scap;   // a parent seldom has fewer survivors than its map may hold
+    for (int n = blocks; n > 0; --n) {
+        int S = 0;
+        while (S + 32 <= Scap && merge_shared_bytes<T>(S + 32, G, threads / 32) <= room(n)) S += 32;
+        if (2 * S >= 3 * G) return S;
+    }
+    return Scap;
 }
 
 // the prefilter's values of component i: pm[k S + i] the mean's u, v, d, pf[k S + i] the
@@ -2018,6 +2041,7 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
 template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
     k_merge(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int cur, int M, int fixed, int S, int over) {
+    chain_wait();
     const int n = over ? min(b.flags[3], prm.N) : prm.N;
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         merge_body<T, K>(prm, b, cur, M, fixed, over ? b.src_tmp[i] : i, S);
@@ -2031,6 +2055,7 @@ template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
     k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int width,
                   int over) {
+    chain_wait<true>();
     const int2 fp = over ? make_int2(blockIdx.x % count, blockIdx.x / count) : map[blockIdx.x];
     const Params& prm = tab.prm[fp.x];
     const Bufs<T>& b = tab.b[fp.x];
@@ -2186,6 +2211,7 @@ inline int weights_threads(int N) { return N >= 1024 ? 1024 : (N + 31) / 32 * 32
 
 template <typename T>
 __global__ void __launch_bounds__(1024) k_weights(__grid_constant__ const Bufs<T> b, int N, int apply) {
+    chain_wait();
     weights_body(N, b.lw, b.loglik, apply, b.scal, b.counters, b.snap, nullptr);
 }
 
@@ -2330,6 +2356,7 @@ __global__ void __launch_bounds__(1024) k_resample(__grid_constant__ const Param
                                                    double* ext_tmp, int* src, int* src_tmp, double* cum, double* scal,
                                                    int* flags, int* idx_out, uint32_t frame, int force,
                                                    double r0_override, unsigned long long* counters, int gather_ext) {
+    chain_wait();
     resample_body(prm, lw, ext, ext_tmp, src, src_tmp, cum, scal, flags, idx_out, frame, force, r0_override, counters,
                   gather_ext != 0);
 }
@@ -2338,12 +2365,14 @@ __global__ void __launch_bounds__(1024) k_resample(__grid_constant__ const Param
 // per state value, ext_tmp[j] = ext[idx[j]], then ext = ext_tmp (when flags[0] says the
 // step resampled; otherwise both return at once)
 __global__ void k_gather_parents(const int* flags, const int* idx, const double* ext, double* ext_tmp, int N) {
+    chain_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (!flags[0] || e >= 12 * N) return;
     const int j = e / 12;
     ext_tmp[e] = ext[12 * idx[j] + (e - 12 * j)];
 }
 __global__ void k_copy_parents(const int* flags, const double* ext_tmp, double* ext, int N) {
+    chain_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (!flags[0] || e >= 12 * N) return;
     ext[e] = ext_tmp[e];
@@ -2354,6 +2383,7 @@ __global__ void k_copy_parents(const int* flags, const double* ext_tmp, double* 
 template <typename T>
 __global__ void __launch_bounds__(1024)
     k_weights_resample(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int apply, uint32_t frame) {
+    chain_wait();
     const double neff = weights_body(prm.N, b.lw, b.loglik, apply, b.scal, b.counters, b.snap, b.cum);
     __syncthreads();
     resample_body(prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal, b.flags, b.resample_idx, frame, 0, -1.0,
@@ -2362,6 +2392,7 @@ __global__ void __launch_bounds__(1024)
 
 template <typename T>
 __global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas) {
+    chain_wait<true>();
     const Bufs<T>& b = tab.b[blockIdx.x];
     const Params& prm = tab.prm[blockIdx.x];
     const FrameArgs& fa = fas[blockIdx.x];
@@ -2377,6 +2408,7 @@ __global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_co
 template <typename T>
 __global__ void k_predict_parents_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map,
                                         int* work) {
+    chain_wait<true>();
     const int2 fp = map[blockIdx.x];
     const Bufs<T>& b = tab.b[fp.x];
     const FrameArgs& fa = fas[fp.x];
