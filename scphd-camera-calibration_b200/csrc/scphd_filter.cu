@@ -12,6 +12,7 @@
 #include <mutex>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <utility>
 #include <vector>
@@ -285,11 +286,47 @@ __global__ void k_reset_src(int* src, int n) {
     if (i < n) src[i] = i;
 }
 
+// the last update's normalisers (rows of Mcap) for the host: FP64, rows of M; a block per parent
+template <typename T> __global__ void k_ell_out(const T* ell, double* out, int M, int Mcap) {
+    const size_t p = blockIdx.x;
+    for (int m = threadIdx.x; m < M; m += blockDim.x) out[p * M + m] = (double)ell[p * Mcap + m];
+}
+
 template <typename T> class Filter final : public scphd_filter {
 public:
     Bufs<T> b{};
     void* arena_ptr = nullptr;
     double* dump = nullptr;   // Gcap x 7 x P: a parent's cloud for the host
+    double* ell_out = nullptr;   // N x Mcap: the normalisers for the host
+    // Results of up to kReadBytes come back through page-locked memory behind h_stage: the copies
+    // are queued and waited for once, where each copy to a caller's pageable array waits for
+    // itself (24 KB of parents' states and weights 36 -> 15 us)
+    static constexpr size_t kReadBytes = 512 * 1024;
+    char* h_read = nullptr;
+    struct Piece {
+        void* to;
+        const void* from;
+        size_t bytes;
+    };
+    scphd_status fetch(std::initializer_list<Piece> pieces) {
+        size_t total = 0;
+        for (const Piece& q : pieces) total += (q.bytes + 15) & ~(size_t)15;
+        const bool staged = total <= kReadBytes;
+        char* at = h_read;
+        for (const Piece& q : pieces) {
+            if (!q.to || !q.bytes) continue;
+            CUDA_TRY(cudaMemcpyAsync(staged ? at : q.to, q.from, q.bytes, cudaMemcpyDeviceToHost, stream));
+            at += (q.bytes + 15) & ~(size_t)15;
+        }
+        CUDA_TRY(cudaStreamSynchronize(stream));
+        at = h_read;
+        for (const Piece& q : pieces) {
+            if (!staged || !q.to || !q.bytes) continue;
+            std::memcpy(q.to, at, q.bytes);
+            at += (q.bytes + 15) & ~(size_t)15;
+        }
+        return SCPHD_OK;
+    }
     size_t merge_smem = 0;       // the full survivor capacity's
     int merge_over_grid = 0;     // blocks of the second merge launch
     struct MergeLaunch { int S = 0; size_t smem = 0; } merge_at[kMergeWidths];   // first launch, by width
@@ -338,6 +375,7 @@ public:
         b.counters = a.take<unsigned long long>(16);
         b.snap = a.take<unsigned long long>(2);
         dump = a.take<double>(G * 7 * prm.P);
+        ell_out = a.take<double>(N * Mc);
         b.fit_n = a.take<int>(N);
         d_stage = a.take<double>(Mc * 3);
     }
@@ -351,7 +389,9 @@ public:
         CUDA_TRY(cudaEventCreate(&merge_ev[0]));
         CUDA_TRY(cudaEventCreate(&merge_ev[1]));
         CUDA_TRY(cudaEventCreateWithFlags(&stage_ev, cudaEventDisableTiming));
-        CUDA_TRY(cudaMallocHost(&h_stage, sizeof(double) * 3 * prm.Mcap));
+        const size_t stage_bytes = (sizeof(double) * 3 * prm.Mcap + 255) & ~(size_t)255;
+        CUDA_TRY(cudaMallocHost(&h_stage, stage_bytes + kReadBytes));
+        h_read = reinterpret_cast<char*>(h_stage) + stage_bytes;
         Arena probe;
         carve(probe);
         void* p = nullptr;
@@ -580,18 +620,15 @@ public:
         stage_end(h);
         if (read_back) {
             int f = 0;
-            CUDA_TRY(cudaMemcpyAsync(&f, b.flags, sizeof(int), cudaMemcpyDeviceToHost, stream));
-            CUDA_TRY(cudaStreamSynchronize(stream));
+            const scphd_status rs = fetch({{&f, b.flags, sizeof(int)}});
+            if (rs != SCPHD_OK) return rs;
             if (resampled) *resampled = f;
         }
         return SCPHD_OK;
     }
 
     scphd_status get_particles(double* st, double* lw) override {
-        const scphd_status s = get_particles_async(st, lw);
-        if (s != SCPHD_OK) return s;
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        return SCPHD_OK;
+        return fetch({{st, b.ext, sizeof(double) * 12 * prm.N}, {lw, b.lw, sizeof(double) * prm.N}});
     }
     scphd_status get_particles_async(double* st, double* lw) override {
         if (st) CUDA_TRY(cudaMemcpyAsync(st, b.ext, sizeof(double) * 12 * prm.N, cudaMemcpyDeviceToHost, stream));
@@ -602,10 +639,7 @@ public:
     scphd_status host_rows(std::vector<int>& src, std::vector<int>& n) {
         src.resize(prm.N);
         n.resize(prm.N);
-        CUDA_TRY(cudaMemcpyAsync(src.data(), b.src, sizeof(int) * prm.N, cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaMemcpyAsync(n.data(), b.map_n[cur], sizeof(int) * prm.N, cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        return SCPHD_OK;
+        return fetch({{src.data(), b.src, sizeof(int) * prm.N}, {n.data(), b.map_n[cur], sizeof(int) * prm.N}});
     }
 
     scphd_status get_map_sizes(int32_t* sizes) override {
@@ -623,9 +657,8 @@ public:
         const int row = src[p], G = n[row];
         std::vector<T> rows((size_t)G * kRow);
         if (G) {
-            CUDA_TRY(cudaMemcpyAsync(rows.data(), b.map[cur] + (size_t)row * prm.Gcap * kRow, sizeof(T) * G * kRow,
-                                     cudaMemcpyDeviceToHost, stream));
-            CUDA_TRY(cudaStreamSynchronize(stream));
+            s = fetch({{rows.data(), b.map[cur] + (size_t)row * prm.Gcap * kRow, sizeof(T) * G * kRow}});
+            if (s != SCPHD_OK) return s;
         }
         const T ps = pending ? (T)prm.ps : T(1);
         for (int j = 0; j < G; ++j) w[j] = (double)(rows[(size_t)j * kRow] * ps);
@@ -642,10 +675,7 @@ public:
         k_map_cloud<T><<<(G * P + 127) / 128, 128, 0, stream>>>(prm, b, cur, dump, d_om, G, pending ? 1 : 0, pending_dt,
                                                                 pending_frame, sample_frame[cur], p);
         LAUNCHED();
-        if (xyz) CUDA_TRY(cudaMemcpyAsync(xyz, dump, sizeof(double) * G * 6 * P, cudaMemcpyDeviceToHost, stream));
-        if (om) CUDA_TRY(cudaMemcpyAsync(om, d_om, sizeof(double) * G * P, cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        return SCPHD_OK;
+        return fetch({{xyz, dump, sizeof(double) * G * 6 * P}, {om, d_om, sizeof(double) * G * P}});
     }
 
     scphd_status get_mixture(int which, int p, double* out, int32_t* count) override {
@@ -689,24 +719,16 @@ public:
     }
 
     scphd_status get_normalizers(double* ell, double* ll) override {
-        if (ell && last_M > 0) {
-            std::vector<T> h((size_t)prm.N * prm.Mcap);
-            CUDA_TRY(cudaMemcpyAsync(h.data(), b.ell, sizeof(T) * h.size(), cudaMemcpyDeviceToHost, stream));
-            CUDA_TRY(cudaStreamSynchronize(stream));
-            for (int p = 0; p < prm.N; ++p)
-                for (int m = 0; m < last_M; ++m) ell[(size_t)p * last_M + m] = (double)h[(size_t)p * prm.Mcap + m];
+        const bool any = ell && last_M > 0;
+        if (any) {
+            k_ell_out<T><<<prm.N, 128, 0, stream>>>(b.ell, ell_out, last_M, prm.Mcap);
+            LAUNCHED();
         }
-        if (ll) {
-            CUDA_TRY(cudaMemcpyAsync(ll, b.loglik, sizeof(double) * prm.N, cudaMemcpyDeviceToHost, stream));
-            CUDA_TRY(cudaStreamSynchronize(stream));
-        }
-        return SCPHD_OK;
+        return fetch({{any ? ell : nullptr, ell_out, sizeof(double) * prm.N * last_M}, {ll, b.loglik, sizeof(double) * prm.N}});
     }
 
     scphd_status get_resample_indices(int32_t* idx) override {
-        CUDA_TRY(cudaMemcpyAsync(idx, b.resample_idx, sizeof(int) * prm.N, cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
-        return SCPHD_OK;
+        return fetch({{idx, b.resample_idx, sizeof(int) * prm.N}});
     }
 
     scphd_status set_state(const double* st, const double* lw, const int32_t* sizes, const double* w,
@@ -744,16 +766,16 @@ public:
 
     scphd_status get_counters(int64_t* c) override {
         unsigned long long h[16];
-        CUDA_TRY(cudaMemcpyAsync(h, b.counters, sizeof(h), cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
+        const scphd_status s = fetch({{h, b.counters, sizeof(h)}});
+        if (s != SCPHD_OK) return s;
         for (int i = 0; i < 16; ++i) c[i] = (int64_t)h[i];
         return SCPHD_OK;
     }
 
     scphd_status check() override {
         std::vector<double> lw(prm.N);
-        CUDA_TRY(cudaMemcpyAsync(lw.data(), b.lw, sizeof(double) * prm.N, cudaMemcpyDeviceToHost, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
+        const scphd_status s = fetch({{lw.data(), b.lw, sizeof(double) * prm.N}});
+        if (s != SCPHD_OK) return s;
         for (double v : lw)
             if (std::isnan(v)) return fail(SCPHD_ERR_NAN, "nan weight detected");
         return SCPHD_OK;
