@@ -548,8 +548,8 @@ public:
             LAUNCHED();
             stage_end(h);
             if (M > 0) {
-                const int bs = sh.lik_full ? likelihood_block(M) : 128;
-                dim3 grid(N, (M + bs - 1) / bs);
+                const int bs = sh.lik_full ? likelihood_block<T>(M) : 128 / kLikPer<T>, per = bs * kLikPer<T>;
+                dim3 grid(N, (M + per - 1) / per);
                 h = stage_begin(2);
                 chained(k_likelihood<T, K>, grid, bs, likelihood_smem_bytes<T>(prm.Gcap, bs), stream, prm, b, cur, M);
                 LAUNCHED();
@@ -1500,7 +1500,7 @@ template <typename T> struct Batch final : scphd_batch {
         std::vector<std::vector<int2>> mp, mpred;
         std::vector<std::vector<int4>> ml;
         stage_off.resize(F);
-        for (int f = 0; f < F; ++f) lik_block = std::max(lik_block, likelihood_block(fs[f]->prm.Mcap));
+        for (int f = 0; f < F; ++f) lik_block = std::max(lik_block, likelihood_block<T>(fs[f]->prm.Mcap));
         for (int first = 0; first < F; first += kBatchSlots) {
             Group g;
             g.first = first;
@@ -1518,7 +1518,7 @@ template <typename T> struct Batch final : scphd_batch {
                 g.tab->b[i] = fl->b;
                 for (int q = 0; q < pr.N; ++q) mp.back().push_back(make_int2(i, q));
                 for (int q = 0; q < pr.N; q += 256) mpred.back().push_back(make_int2(i, q));
-                const int mb = (pr.Mcap + lik_block - 1) / lik_block;
+                const int per = lik_block * kLikPer<T>, mb = (pr.Mcap + per - 1) / per;
                 for (int q = 0; q < pr.N; ++q)
                     for (int k = 0; k < mb; ++k) ml.back().push_back(make_int4(i, q, k, 0));
                 stage_off[first + i] = stage_total;

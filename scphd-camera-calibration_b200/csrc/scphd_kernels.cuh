@@ -94,7 +94,7 @@ struct FrameArgs {
 
 // Up to kBatchSlots filters of a batch per launch: their constants and buffers as
 // one kernel parameter (read-only parameter space, like a single filter's Params;
-// 32 x 824 bytes fits the 32 KB parameter limit).  Each frame's per-filter
+// 32 x 904 bytes fits the 32 KB parameter limit).  Each frame's per-filter
 // arguments are a separate FrameArgs array in global memory.
 constexpr int kBatchSlots = 32;
 template <typename T> struct SlotTable {
@@ -777,20 +777,38 @@ __global__ void __launch_bounds__(kPrepThreads)
 // Normaliser ell_{p,m} = logsumexp_j(log w_{j,m}) (+) log(M w0 + kappa)
 // (.cu:1729-1768) and survivor compaction: w_{j,m} = exp(log w - ell) >= min_weight
 // with a PD posterior (updateKernel, kernels.cu:622-657), births likewise.
-// One thread per measurement; a block covers the frame's measurements (a multiple
-// of 32 threads, up to 1024; more measurements take more blocks) and stages the
+// A thread per measurement, or per two in FP32; a block covers the frame's measurements
+// (up to 1024, by a multiple of 32 threads; more take more blocks) and stages the
 // parent's Gaussian terms once in shared memory for both passes.  Since ell >= bpc =
 // log(M w0 + kappa) (the sum inside the log holds exp(0) = 1 around its larger term),
 // a pair with log w < bpc + log(min_weight) - 1 can never reach min_weight; the first
 // pass remembers the pairs above that bound (up to kLikCand per measurement) and the
 // survivor pass evaluates only those (all pairs again if the list overflowed).
-constexpr int kLikCand = 16;   // candidate survivors remembered per measurement
-template <typename T> __host__ __device__ inline size_t likelihood_smem_bytes(int Gcap, int block) {
-    return (size_t)Gcap * kLikTerms * sizeof(T) + (size_t)block * kLikCand * sizeof(int);
+//
+// FP32 takes two Gaussians at a time in packed operations: their terms are staged side by
+// side, the measurement is doubled in registers, and the exponentials are summed one by one,
+// in the Gaussians' order (the one-by-one form's normalisers bit for bit); a thread has two
+// measurements, so that terms read from shared memory serve four pairs.  Per launch of 4096
+// parents x 256 Gaussians: 0.188 ms one by one, 0.175 in pairs, 0.169 with two measurements.
+// FP64 takes Gaussians and measurements one by one.
+constexpr int kLikCand = 15;   // candidate survivors remembered per measurement
+template <typename T> constexpr int kLikPer = sizeof(T) == 4 ? 2 : 1;          // measurements of a thread
+template <typename T> constexpr int kLikThreads = 1024 / kLikPer<T>;            // of a block, at most
+typedef unsigned short LikIndex;   // shared memory holds fewer than 2^16 Gaussians' terms
+// two Gaussians' log-constants, S^-1, negated means and pD flags, the even one's low; behind
+// the last Gaussian of an odd map its own terms again with log-constant -inf
+constexpr int kLikPair = 12;   // 16-byte pieces
+constexpr int kLpA = 1, kLpMean = 7, kLpFlag = 10;
+template <typename T> __host__ __device__ inline int likelihood_rows(int Gcap) {
+    return sizeof(T) == 4 ? (Gcap + 1) / 2 * 2 : Gcap;
 }
-__host__ __device__ inline int likelihood_block(int M) {
-    const int r = (M + 31) / 32 * 32;
-    return r < 32 ? 32 : (r > 1024 ? 1024 : r);
+template <typename T> __host__ __device__ inline size_t likelihood_smem_bytes(int Gcap, int block) {
+    return (size_t)likelihood_rows<T>(Gcap) * kLikTerms * sizeof(T) +
+           (size_t)block * kLikPer<T> * kLikCand * sizeof(LikIndex);
+}
+template <typename T> __host__ __device__ inline int likelihood_block(int M) {
+    const int r = ((M + kLikPer<T> - 1) / kLikPer<T> + 31) / 32 * 32;
+    return r < 32 ? 32 : (r > kLikThreads<T> ? kLikThreads<T> : r);
 }
 
 __device__ __forceinline__ void load_terms(const float* src, float* t) {
@@ -820,32 +838,81 @@ __device__ __forceinline__ void store_terms(double* dst, const double* t) {
     for (int i = 0; i < 6; ++i) v[i] = make_double2(t[2 * i], t[2 * i + 1]);
 }
 
+// Gaussian k's terms from its pair, in the rows' layout
+__device__ __forceinline__ void load_paired(const float* s_terms, int k, float* t) {
+    const float* q = s_terms + (size_t)(k >> 1) * (2 * kLikPair) + (k & 1);
+    t[0] = q[0];
+    t[1] = q[2 * kLpFlag];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) t[2 + i] = q[2 * (kLpA + i)];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) t[8 + i] = -q[2 * (kLpMean + i)];
+}
+__device__ __forceinline__ void load_paired(const double* s_terms, int k, double* t) {
+    load_terms(s_terms + (size_t)k * kLikTerms, t);
+}
+// log2_term of the two Gaussians of a pair
+template <int K> __device__ __forceinline__ F2 log2_term_pair(const F2* r, const F2* z) {
+    const F2* A = r + kLpA;
+    const F2 n0 = f2_add(z[0], r[kLpMean]), n1 = f2_add(z[1], r[kLpMean + 1]);
+    if (K == 2) return f2_fma(n1, f2_mul(A[2], n1), f2_fma(n0, f2_fma(A[1], n1, f2_mul(A[0], n0)), r[0]));
+    const F2 n2 = f2_add(z[2], r[kLpMean + 2]);
+    const F2 u0 = f2_fma(A[3], n2, f2_fma(A[1], n1, f2_mul(A[0], n0)));
+    const F2 u1 = f2_fma(A[4], n2, f2_mul(A[2], n1));
+    return f2_fma(n2, f2_mul(A[5], n2), f2_fma(n1, u1, f2_fma(n0, u0, r[0])));
+}
+
 template <typename T, int K>
 __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>& b, int cur, int M, int p,
                                                 int mblock, T* s_terms) {
-    const int m = mblock * blockDim.x + threadIdx.x;
+    // the thread's measurements: m0, m0 + blockDim.x
+    constexpr int kPer = kLikPer<T>;
+    const int m0 = mblock * kPer * (int)blockDim.x + threadIdx.x;
     const int G = min(b.map_n[cur][b.src[p]], prm.Gcap);
     // per Gaussian: c (-inf for a non-PD posterior), pD flag, S^-1, mean, pad -- the
     // compact rows k_prep wrote, copied into shared memory in 16-byte pieces
     T cm = tneg_inf<T>();
-    for (int jj = threadIdx.x; jj < G; jj += blockDim.x) {
-        T t[kLikTerms];
-        load_terms(b.lik + ((size_t)p * prm.Gcap + jj) * kLikTerms, t);
-        cm = t[0] > cm ? t[0] : cm;
-        store_terms(s_terms + (size_t)jj * kLikTerms, t);
+    if constexpr (sizeof(T) == 4) {
+        for (int q = threadIdx.x; q < (G + 1) / 2; q += blockDim.x) {
+            float t[kLikTerms], u[kLikTerms];
+            const float* rows = b.lik + ((size_t)p * prm.Gcap + 2 * q) * kLikTerms;
+            const bool two = 2 * q + 1 < G;
+            load_terms(rows, t);
+            load_terms(two ? rows + kLikTerms : rows, u);
+            if (!two) u[0] = tneg_inf<float>();
+            cm = fmaxf(cm, fmaxf(t[0], u[0]));
+            float4* to = reinterpret_cast<float4*>(s_terms + (size_t)q * (2 * kLikPair));
+            to[0] = make_float4(t[0], u[0], t[2], u[2]);
+            to[1] = make_float4(t[3], u[3], t[4], u[4]);
+            to[2] = make_float4(t[5], u[5], t[6], u[6]);
+            to[3] = make_float4(t[7], u[7], -t[8], -u[8]);
+            to[4] = make_float4(-t[9], -u[9], -t[10], -u[10]);
+            to[5] = make_float4(t[1], u[1], 0.0f, 0.0f);
+        }
+    } else {
+        for (int jj = threadIdx.x; jj < G; jj += blockDim.x) {
+            T t[kLikTerms];
+            load_terms(b.lik + ((size_t)p * prm.Gcap + jj) * kLikTerms, t);
+            cm = t[0] > cm ? t[0] : cm;
+            store_terms(s_terms + (size_t)jj * kLikTerms, t);
+        }
     }
-    T zm[3] = {0, 0, 0};
-    if (m < M) {
+    T zm[kPer][3] = {};
 #pragma unroll
-        for (int a2 = 0; a2 < K; ++a2) zm[a2] = b.z[m * 3 + a2];
+    for (int i = 0; i < kPer; ++i) {
+        const int m = m0 + i * (int)blockDim.x;
+        if (m < M) {
+#pragma unroll
+            for (int a2 = 0; a2 < K; ++a2) zm[i][a2] = b.z[m * 3 + a2];
+        }
     }
     // the pair terms' base: log2 in FP32 (log2_term on the rows k_prep scaled), ln in FP64;
     // sc = the factor from ln to that base, ic its inverse
     constexpr bool kB2 = sizeof(T) == 4;
     const T sc = kB2 ? T(kLog2e) : T(1), ic = kB2 ? T(kLn2) : T(1);
-    auto pair_term = [&](const T* t) -> T {
-        if constexpr (kB2) return log2_term<K>(t[0], t + 2, t + 8, zm);
-        else return log_term<T, K>(t[0], t + 2, t + 8, zm);
+    auto pair_term = [&](const T* t, const T* z) -> T {
+        if constexpr (kB2) return log2_term<K>(t[0], t + 2, t + 8, z);
+        else return log_term<T, K>(t[0], t + 2, t + 8, z);
     };
     auto exp_w = [&](T x) -> T {   // base^x for the normaliser sums and survivor weights
         if constexpr (kB2) return exp2_approx(x);
@@ -854,8 +921,12 @@ __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>
     const T bpc = (T)log((double)M * prm.w0 + prm.kappa);   // ln of the birth + clutter term
     const T bpc_w = bpc * sc;
     const T cand_min = (bpc + (T)log(prm.min_weight) - T(1)) * sc;
-    int* s_cand = reinterpret_cast<int*>(s_terms + (size_t)prm.Gcap * kLikTerms);   // [slot][thread]
-    int n_cand = 0;
+    LikIndex* s_cand = reinterpret_cast<LikIndex*>(s_terms + (size_t)likelihood_rows<T>(prm.Gcap) * kLikTerms);   // [slot][measurement]
+    int n_cand[kPer] = {};
+    auto candidate = [&](int i, int k) {
+        if (n_cand[i] < kLikCand) s_cand[(n_cand[i] * kPer + i) * blockDim.x + threadIdx.x] = (LikIndex)k;
+        ++n_cand[i];
+    };
     // largest log-constant of the parent: lt_j <= c_j, since the quadratic form is >= 0
     __shared__ T s_cm[32];
 #pragma unroll
@@ -874,42 +945,68 @@ __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>
     // tied weights with it.  (FP32 values are in base 2 here, the limits scaled alike.)
     const T s0 = cm > bpc_w ? cm : bpc_w;
     const bool fixed_shift = kB2 && !(cm - bpc_w > T(60) * sc);
-    T mx = tneg_inf<T>(), acc = 0;
-    if (m < M) {
-        if (fixed_shift) {
-            for (int k = 0; k < G; ++k) {
-                T t[kLikTerms];
-                load_terms(s_terms + (size_t)k * kLikTerms, t);
-                const T lt = pair_term(t);   // -inf for a non-PD posterior
-                acc += exp_w(lt - s0);
-                if (lt >= cand_min) {
-                    if (n_cand < kLikCand) s_cand[n_cand * blockDim.x + threadIdx.x] = k;
-                    ++n_cand;
+    T mx[kPer], acc[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) mx[i] = tneg_inf<T>(), acc[i] = 0;
+    if constexpr (kB2) {
+        if (fixed_shift && m0 < M) {
+            F2 z2[kPer][3];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+#pragma unroll
+                for (int a2 = 0; a2 < 3; ++a2) z2[i][a2] = f2_dup(zm[i][a2]);
+            }
+            const F2 shift = f2_dup(-s0);
+            for (int k = 0; k < G; k += 2) {
+                const ulonglong2* from = reinterpret_cast<const ulonglong2*>(s_terms + (size_t)k * kLikPair);
+                F2 r[kLikPair];
+#pragma unroll
+                for (int i = 0; i < kLikPair / 2; ++i) {
+                    const ulonglong2 v = from[i];
+                    r[2 * i] = v.x;
+                    r[2 * i + 1] = v.y;
+                }
+                F2 lt[kPer];   // -inf for a non-PD posterior
+#pragma unroll
+                for (int i = 0; i < kPer; ++i) {
+                    lt[i] = log2_term_pair<K>(r, z2[i]);
+                    const F2 x = f2_add(lt[i], shift);
+                    acc[i] += exp_w(f2_lo(x));
+                    acc[i] += exp_w(f2_hi(x));
+                }
+#pragma unroll
+                for (int i = 0; i < kPer; ++i) {
+                    if (fmaxf(f2_lo(lt[i]), f2_hi(lt[i])) >= cand_min) {
+                        if (f2_lo(lt[i]) >= cand_min) candidate(i, k);
+                        if (f2_hi(lt[i]) >= cand_min && k + 1 < G) candidate(i, k + 1);
+                    }
                 }
             }
-        } else {
+        }
+    }
+    if (!fixed_shift) {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            if (m0 + i * (int)blockDim.x >= M) continue;
             for (int k = 0; k < G; ++k) {
                 T t[kLikTerms];
-                load_terms(s_terms + (size_t)k * kLikTerms, t);
+                load_paired(s_terms, k, t);
                 const T c = t[0];
                 if (!(c > tneg_inf<T>())) continue;
-                const T lt = pair_term(t);
+                const T lt = pair_term(t, zm[i]);
                 // FP64 exponentials that cannot change the sum are not taken (most pairs are far
                 // apart; 0.73 -> 0.40 ms at 4096 parents x 256 Gaussians): the sum holds its
                 // largest term as 1, so a term below e^-38 < 2^-54 is rounded off, and so is what
                 // a new largest term more than 60 above scales down (at most G 2^-86)
-                if (lt > mx) {   // online log-sum-exp
-                    const T d = mx - lt;
-                    acc = !kB2 && d < T(-60) ? T(1) : acc * exp_w(d) + T(1);
-                    mx = lt;
+                if (lt > mx[i]) {   // online log-sum-exp
+                    const T d = mx[i] - lt;
+                    acc[i] = !kB2 && d < T(-60) ? T(1) : acc[i] * exp_w(d) + T(1);
+                    mx[i] = lt;
                 } else {
-                    const T d = lt - mx;
-                    if (kB2 || !(d <= T(-38))) acc += exp_w(d);
+                    const T d = lt - mx[i];
+                    if (kB2 || !(d <= T(-38))) acc[i] += exp_w(d);
                 }
-                if (lt >= cand_min) {
-                    if (n_cand < kLikCand) s_cand[n_cand * blockDim.x + threadIdx.x] = k;
-                    ++n_cand;
-                }
+                if (lt >= cand_min) candidate(i, k);
             }
         }
     }
@@ -922,66 +1019,70 @@ __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>
         if constexpr (kB2) return exp2f(x);
         else return texp(x);
     };
-    T ell_w = bpc_w;
-    if (m < M && fixed_shift) {
-        ell_w = s0 + log_b(acc + exp_b(bpc_w - s0));
-    } else if (m < M && mx > tneg_inf<T>()) {
-        // evaluated around the larger of the two
-        T big = mx > bpc_w ? mx : bpc_w;
-        ell_w = big + log_b(acc * exp_b(mx - big) + exp_b(bpc_w - big));
-    }
-    const T ell = kB2 ? ell_w * ic : ell_w;
-    if (m < M) b.ell[(size_t)p * prm.Mcap + m] = ell;
-    // survivors among the candidates (or all pairs, if the list overflowed)
     const T minw = (T)prm.min_weight;
     const unsigned lane = threadIdx.x & 31;
-    if (m < M) {
-        const bool all = n_cand > kLikCand;
-        const int nk = all ? G : n_cand;
-        for (int q = 0; q < nk; ++q) {
-            const int k = all ? q : s_cand[q * blockDim.x + threadIdx.x];
-            T t[kLikTerms];
-            load_terms(s_terms + (size_t)k * kLikTerms, t);
-            const T c = t[0];
-            if (!(c > tneg_inf<T>() && t[1] > T(0))) continue;
-            const T w = exp_w(pair_term(t) - ell_w);
-            if (w >= minw) {
-                const int slot = atomicAdd(&b.surv_n[p], 1);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int m = m0 + i * (int)blockDim.x;
+        T ell_w = bpc_w;
+        if (m < M && fixed_shift) {
+            ell_w = s0 + log_b(acc[i] + exp_b(bpc_w - s0));
+        } else if (m < M && mx[i] > tneg_inf<T>()) {
+            // evaluated around the larger of the two
+            T big = mx[i] > bpc_w ? mx[i] : bpc_w;
+            ell_w = big + log_b(acc[i] * exp_b(mx[i] - big) + exp_b(bpc_w - big));
+        }
+        const T ell = kB2 ? ell_w * ic : ell_w;
+        if (m < M) b.ell[(size_t)p * prm.Mcap + m] = ell;
+        // survivors among the candidates (or all pairs, if the list overflowed)
+        if (m < M) {
+            const bool all = n_cand[i] > kLikCand;
+            const int nk = all ? G : n_cand[i];
+            for (int q = 0; q < nk; ++q) {
+                const int k = all ? q : s_cand[(q * kPer + i) * blockDim.x + threadIdx.x];
+                T t[kLikTerms];
+                load_paired(s_terms, k, t);
+                const T c = t[0];
+                if (!(c > tneg_inf<T>() && t[1] > T(0))) continue;
+                const T w = exp_w(pair_term(t, zm[i]) - ell_w);
+                if (w >= minw) {
+                    const int slot = atomicAdd(&b.surv_n[p], 1);
+                    if (slot < prm.Scap) {
+                        b.surv_r[(size_t)p * prm.Scap + slot] = m * G + k;
+                        b.surv_w[(size_t)p * prm.Scap + slot] = w;
+                    } else {
+                        atomicAdd(&b.counters[1], 1ull);
+                    }
+                }
+            }
+        }
+        // birth term of measurement m (always PD)
+        bool keep = false;
+        T wb = 0;
+        if (m < M) {
+            wb = texp((T)log(prm.w0) - ell);
+            keep = wb >= minw;
+        }
+        unsigned mask = __ballot_sync(0xffffffffu, keep);
+        if (mask) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&b.surv_n[p], __popc(mask));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (keep) {
+                int slot = base + __popc(mask & ((1u << lane) - 1u));
                 if (slot < prm.Scap) {
-                    b.surv_r[(size_t)p * prm.Scap + slot] = m * G + k;
-                    b.surv_w[(size_t)p * prm.Scap + slot] = w;
+                    b.surv_r[(size_t)p * prm.Scap + slot] = G * M + m;
+                    b.surv_w[(size_t)p * prm.Scap + slot] = wb;
                 } else {
                     atomicAdd(&b.counters[1], 1ull);
                 }
             }
         }
     }
-    // birth term of measurement m (always PD)
-    bool keep = false;
-    T wb = 0;
-    if (m < M) {
-        wb = texp((T)log(prm.w0) - ell);
-        keep = wb >= minw;
-    }
-    unsigned mask = __ballot_sync(0xffffffffu, keep);
-    if (mask) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&b.surv_n[p], __popc(mask));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (keep) {
-            int slot = base + __popc(mask & ((1u << lane) - 1u));
-            if (slot < prm.Scap) {
-                b.surv_r[(size_t)p * prm.Scap + slot] = G * M + m;
-                b.surv_w[(size_t)p * prm.Scap + slot] = wb;
-            } else {
-                atomicAdd(&b.counters[1], 1ull);
-            }
-        }
-    }
 }
 
 template <typename T, int K>
-__global__ void __launch_bounds__(1024) k_likelihood(__grid_constant__ const Params prm,
+__global__ void __launch_bounds__(kLikThreads<T>) k_likelihood(__grid_constant__ const Params prm,
                                                      __grid_constant__ const Bufs<T> b, int cur, int M) {
     chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_lik[];
@@ -990,13 +1091,13 @@ __global__ void __launch_bounds__(1024) k_likelihood(__grid_constant__ const Par
 
 // map entry: (filter, parent, measurement block); blocks past a filter's M exit
 template <typename T, int K>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(kLikThreads<T>)
     k_likelihood_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int4* map) {
     chain_wait<true>();
     extern __shared__ __align__(16) unsigned char dsm_lik[];
     const int4 e = map[blockIdx.x];
     const int M = fas[e.x].M;
-    if (e.z * (int)blockDim.x >= M) return;
+    if (e.z * kLikPer<T> * (int)blockDim.x >= M) return;
     likelihood_body<T, K>(tab.prm[e.x], tab.b[e.x], fas[e.x].cur, M, e.y, e.z, reinterpret_cast<T*>(dsm_lik));
 }
 
@@ -2094,7 +2195,7 @@ __device__ __forceinline__ void fused_parent(const Params& prm, const Bufs<T>& b
                          nullptr, nullptr, p, 0, 1, reinterpret_cast<T*>(smem));
     __syncthreads();
     prep_body<T, K>(prm, b, fa.cur, p, reinterpret_cast<T*>(smem));
-    for (int mb = 0; mb * (int)blockDim.x < fa.M; ++mb) {
+    for (int mb = 0; mb * kLikPer<T> * (int)blockDim.x < fa.M; ++mb) {
         likelihood_body<T, K>(prm, b, fa.cur, fa.M, p, mb, reinterpret_cast<T*>(smem));
         __syncthreads();
     }
