@@ -442,7 +442,7 @@ def run_b200(args):
             slots = 148 * 4 * clk["sm_mhz"] * 1e6 * avg_ms / 1e3
             compute["issue"] = {"warp_instructions_per_launch": inst, "issue_slots_per_launch": slots,
                                 "frac": inst / slots,
-                                "instructions_source": "profiles/k_cloud_fit_plain_c1_512parents.md"}
+                                "instructions_source": "profiles/traffic.json"}
 
     cpu = None
     if world == 1 and not args.no_cpu_baseline:

@@ -208,10 +208,10 @@ scphd_status scphd_get_launch_shapes(scphd_filter* f, int32_t* merge_threads, in
 scphd_status scphd_set_fused(scphd_filter* f, int32_t mode);
 scphd_status scphd_get_fused(scphd_filter* f, int32_t* fused);
 
-/* Cloud-fit tiling: blocks per parent (1, 2 or 4).  Each block has 4 warps in FP32, 8 in
- * FP64, and the parent's daughter Gaussians are dealt out over the warps of all its
- * blocks, so 2 or 4 blocks per parent fill the GPU when a filter has few parents (256
- * blocks leave half of the 148 SMs x 4 block slots of FP32 idle).  By default the
+/* Cloud-fit tiling: blocks per parent (1, 2 or 4).  Each block has 4 warps and
+ * the parent's daughter Gaussians are dealt out over the warps of all its blocks, so 2 or
+ * 4 blocks per parent fill the GPU when a filter has few parents (256 blocks leave more
+ * than half of the 148 SMs x 4 block slots of FP32, x 5 of FP64, idle).  By default the
  * updates with measurements after the first 16 (when the maps have grown) time the
  * cloud-fit launch at each split (twice) and keep the fastest; until then the split is
  * 1.  scphd_set_fit_split fixes one (and ends that tuning),
