@@ -1384,7 +1384,7 @@ template <typename T> struct MergeScratch {
     int* lab;             // S: union-find parent, then the component's root
     int* cidx;            // S: component index of a root; later the queue of large components
     int* start;           // S + 1: member range of each component in perm
-    int* fill;            // S: member ranks within a component, then scratch of the large components
+    int* fill;            // S: member ranks within a component
     int* perm;            // survivors grouped by component (first: survivors in u order)
     uint32_t* masks;      // (blockDim/32) x nchunk member masks
     int nchunk;
@@ -1820,14 +1820,27 @@ __device__ int merge_components(const View& v, const T* s_w, const int* s_r, int
         const int s0 = ms.start[c], cnt = ms.start[c + 1] - s0;
         int* mem = ms.perm + s0;
         const int nch = (cnt + 31) >> 5;
-        for (int k = lane; k < cnt; k += 32) {   // ascending: each member to its rank, by way of fill
-            const int x = mem[k];
-            int rank = 0;
-            for (int q2 = 0; q2 < cnt; ++q2) rank += mem[q2] < x;
-            ms.fill[s0 + rank] = x;
-        }
+        // ascending: the members marked in a bit per survivor (this warp's mask words, free here)
+        // and listed from the bits.  (Counting each one's smaller members took cnt^2 / 32 steps:
+        // 22 us of a merge of 231 survivors in one component, a fifth of one of 1270.)
+        const int nw = (n + 31) >> 5;
+        for (int w = lane; w < nw; w += 32) masks[w] = 0u;
         __syncwarp();
-        for (int k = lane; k < cnt; k += 32) mem[k] = ms.fill[s0 + k];
+        for (int k = lane; k < cnt; k += 32) atomicOr(&masks[mem[k] >> 5], 1u << (mem[k] & 31));
+        __syncwarp();
+        for (int w0 = 0, base = 0; w0 < nw; w0 += 32) {
+            uint32_t bits = w0 + lane < nw ? masks[w0 + lane] : 0u;
+            int at = __popc(bits);   // inclusive sum over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += x;
+            }
+            const int total = __shfl_sync(0xffffffffu, at, 31);
+            at += base - __popc(bits);
+            base += total;
+            for (; bits; bits &= bits - 1) mem[at++] = (w0 + lane) * 32 + __ffs(bits) - 1;
+        }
         __syncwarp();
         int next = 0;
         while (true) {
