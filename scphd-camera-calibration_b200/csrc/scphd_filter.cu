@@ -1412,7 +1412,10 @@ template <typename T> struct Batch final : scphd_batch {
         int4* map_lik = nullptr;    int n_lik = 0;
         int* work = nullptr;            // the fused update's work counter
         bool fit_p = false;             // every member has kFitP samples per feature
-        int merge_over[3] = {0, 0, 0};  // blocks per filter of the second merge launch, by width (0: none needed)
+        // by merge width: the first merge launch's shared memory (Params::Ssm), and the blocks of
+        // the second (0: none needed)
+        size_t merge_first_smem[3] = {0, 0, 0};
+        int merge_over[3] = {0, 0, 0};
     };
     int K = 3;
     bool use_graph = false;
@@ -1429,7 +1432,6 @@ template <typename T> struct Batch final : scphd_batch {
     std::vector<size_t> stage_off;
     size_t stage_total = 0;
     size_t merge_smem = 0;       // the members' full survivor capacities
-    size_t merge_first_smem[3] = {0, 0, 0};   // the first launch's (Params::Ssm), by width
     size_t merge_need = 0;       // the limit's (merge_limit_bytes)
     size_t fit_smem = 0;
     size_t lik_smem = 0;
@@ -1525,13 +1527,6 @@ template <typename T> struct Batch final : scphd_batch {
                 stage_total += 3 * (size_t)pr.Mcap;
                 merge_need = std::max(merge_need, merge_limit_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
                 merge_smem = std::max(merge_smem, merge_shared_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
-                for (int w = 0; w < kPaths; ++w) {
-                    const int threads = merge_widths[w];
-                    const int S = merge_launch_cap<T>(pr.Scap, pr.Gcap, threads, kMergeBlocks<T> * (kMergeThreads / threads));
-                    g.tab->prm[i].Ssm[w] = S;
-                    merge_first_smem[w] = std::max(merge_first_smem[w], merge_shared_bytes<T>(S, pr.Gcap, threads / 32));
-                    if (S < pr.Scap) g.merge_over[w] = std::max(g.merge_over[w], std::min(pr.N, 16));
-                }
                 fit_smem = std::max(fit_smem, fit_kernel_smem_bytes<T>(pr.P));
                 fused_smem = std::max(fused_smem, fused_smem_bytes<T>(pr.P, pr.Gcap, pr.Scap));
                 lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block));
@@ -1594,6 +1589,26 @@ template <typename T> struct Batch final : scphd_batch {
             CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 3>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_prep_batch<T, 3>));
         }
+        {
+            // merge launches: a group whose parents are all resident at the full capacity takes one
+            // launch, like a single filter; the second launch of a larger one fills the GPU
+            const void* fn = K == 2 ? (const void*)k_merge_batch<T, 2> : (const void*)k_merge_batch<T, 3>;
+            int dev = 0, nsm = 0, occ = 0;
+            CUDA_TRY(cudaGetDevice(&dev));
+            CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kMergeThreads, merge_smem));
+            for (Group& g : groups)
+                for (int w = 0; w < kPaths; ++w) {
+                    const int threads = merge_widths[w], blocks = kMergeBlocks<T> * (kMergeThreads / threads);
+                    for (int i = 0; i < g.count; ++i) {
+                        Params& pr = g.tab->prm[i];
+                        pr.Ssm[w] = g.n_parent <= nsm * occ ? pr.Scap : merge_launch_cap<T>(pr.Scap, pr.Gcap, threads, blocks);
+                        g.merge_first_smem[w] =
+                            std::max(g.merge_first_smem[w], merge_shared_bytes<T>(pr.Ssm[w], pr.Gcap, threads / 32));
+                        if (pr.Ssm[w] < pr.Scap) g.merge_over[w] = nsm * occ;
+                    }
+                }
+        }
         // members now issue on the batch stream
         for (scphd_filter* f : fs) {
             CUDA_TRY(cudaStreamSynchronize(f->stream));
@@ -1646,12 +1661,14 @@ template <typename T> struct Batch final : scphd_batch {
             }
             if (timed) CUDA_TRY(cudaEventRecord(tune_ev[0], stream));
             for (const Group& g : groups) {
-                chained(k_merge_batch<T, KK>, g.n_parent, merge_widths[pth], merge_first_smem[pth], stream, *g.tab, d_fa + g.first, g.map_parent, g.count, pth, 0);
+                chained(k_merge_batch<T, KK>, g.n_parent, merge_widths[pth], g.merge_first_smem[pth], stream, *g.tab,
+                        d_fa + g.first, g.map_parent, g.count, pth, 0);
                 LAUNCHED();
             }
             for (const Group& g : groups) {
                 if (!g.merge_over[pth]) continue;
-                chained(k_merge_batch<T, KK>, g.count * g.merge_over[pth], kMergeThreads, merge_smem, stream, *g.tab, d_fa + g.first, g.map_parent, g.count, pth, 1);
+                chained(k_merge_batch<T, KK>, g.merge_over[pth], kMergeThreads, merge_smem, stream, *g.tab, d_fa + g.first,
+                        g.map_parent, g.count, pth, 1);
                 LAUNCHED();
             }
             if (timed) {

@@ -333,7 +333,7 @@ __device__ __forceinline__ void cloud_fit_f32_body(const Params& prm, const Bufs
         tab.meas[4] = f2_dup(nfxB);
     }
     if (threadIdx.x == 0) {
-        if (p == 0 && c == 0) b.flags[3] = 0;   // no parent listed for a second merge launch yet
+        if (p == 0 && c == 0) b.flags[3] = b.flags[1] = 0;   // no parent listed for a second merge launch yet
         double zero[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
         const Pose<float> pu = make_pose<float>(fixed ? zero : b.ext + 12 * p);
 #pragma unroll

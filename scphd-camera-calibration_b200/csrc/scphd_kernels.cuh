@@ -75,7 +75,7 @@ template <typename T> struct Bufs {
     double* loglik;     // N
     double* cum;        // N resampling prefix
     double* scal;       // [0] neff
-    int* flags;         // [0] resampled, [2] fused work counter, [3] parents listed for the second merge launch
+    int* flags;         // [0] resampled, [2] fused work counter, [3] parents listed for the second merge launch, [1] taken by it
     int* resample_idx;  // N
     unsigned long long* counters;   // 16
     unsigned long long* snap;       // counters [6], [7] as the last update left them
@@ -328,7 +328,7 @@ __device__ __forceinline__ void cloud_fit_body(const Params& prm, const Bufs<T>&
     // the two poses (FP64 rotation terms) by threads of two warps, side by side
     if (threadIdx.x == 32) pose_src = make_pose<T>(b.map_ext[cur] + 12 * row);
     if (threadIdx.x == 0) {
-        if (p == 0 && c == 0) b.flags[3] = 0;   // no parent listed for a second merge launch yet
+        if (p == 0 && c == 0) b.flags[3] = b.flags[1] = 0;   // no parent listed for a second merge launch yet
         double zero[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
         pose_upd = make_pose<T>(fixed ? zero : b.ext + 12 * p);
         if (c == 0) {
@@ -2150,33 +2150,69 @@ __device__ __forceinline__ void merge_body(const Params& prm, const Bufs<T>& b, 
     }
 }
 
-// over = 0: block p merges parent p, survivor capacity S; over = 1: the listed parents, at
-// the full capacity, dealt out over the blocks
+// over = 0: block p merges parent p, survivor capacity S; over = 1: the listed parents, at the
+// full capacity, each taken by the next free block (flags[1] counts them: dealt out beforehand,
+// a last round of a grid of 148 blocks is nearly empty)
 template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
     k_merge(__grid_constant__ const Params prm, __grid_constant__ const Bufs<T> b, int cur, int M, int fixed, int S, int over) {
     chain_wait();
-    const int n = over ? min(b.flags[3], prm.N) : prm.N;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
-        merge_body<T, K>(prm, b, cur, M, fixed, over ? b.src_tmp[i] : i, S);
+    __shared__ int s_item;
+    const int n = over ? min(b.flags[3], prm.N) : 1;
+    for (int k = 0; k < n; ++k) {
+        int i = blockIdx.x;
+        if (over) {
+            if (threadIdx.x == 0) s_item = atomicAdd(b.flags + 1, 1);
+            __syncthreads();
+            if (s_item >= n) return;
+            i = b.src_tmp[s_item];
+        }
+        merge_body<T, K>(prm, b, cur, M, fixed, i, S);
         __syncthreads();
     }
 }
 
-// over = 0: a block per (filter, parent) of the map; over = 1: blockIdx.x % count is the
-// filter, its listed parents are dealt out over that filter's blocks
+// over = 0: a block per (filter, parent) of the map; over = 1: the group's listed parents, filter
+// by filter, each taken by the next free block of the whole grid
 template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
     k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int width,
                   int over) {
     chain_wait<true>();
-    const int2 fp = over ? make_int2(blockIdx.x % count, blockIdx.x / count) : map[blockIdx.x];
-    const Params& prm = tab.prm[fp.x];
-    const Bufs<T>& b = tab.b[fp.x];
-    const FrameArgs fa = fas[fp.x];
-    const int n = over ? min(b.flags[3], prm.N) : fp.y + 1, step = over ? gridDim.x / count : 1;
-    for (int i = fp.y; i < n; i += step) {
-        merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, over ? b.src_tmp[i] : i, over ? prm.Scap : prm.Ssm[width]);
+    __shared__ int s_item;
+    __shared__ unsigned s_listed;
+    int2 fp = make_int2(0, 0);
+    unsigned todo = 1u;   // filters with listed parents left
+    if (over) {
+        if (threadIdx.x < 32) {
+            const unsigned listed =
+                __ballot_sync(0xffffffffu, (int)threadIdx.x < count && tab.b[threadIdx.x & (kBatchSlots - 1)].flags[3] > 0);
+            if (threadIdx.x == 0) s_listed = listed;
+        }
+        __syncthreads();
+        todo = s_listed;
+    } else {
+        fp = map[blockIdx.x];
+    }
+    while (todo) {
+        if (over) fp.x = __ffs(todo) - 1;
+        const Params& prm = tab.prm[fp.x];
+        const Bufs<T>& b = tab.b[fp.x];
+        if (over) {
+            if (threadIdx.x == 0) s_item = atomicAdd(b.flags + 1, 1);
+            __syncthreads();
+            const int item = s_item;
+            __syncthreads();
+            if (item >= min(b.flags[3], prm.N)) {
+                todo &= todo - 1;
+                continue;
+            }
+            fp.y = b.src_tmp[item];
+        } else {
+            todo = 0u;
+        }
+        const FrameArgs fa = fas[fp.x];
+        merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, fp.y, over ? prm.Scap : prm.Ssm[width]);
         __syncthreads();
     }
 }
