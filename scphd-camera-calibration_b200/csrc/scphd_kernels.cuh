@@ -105,13 +105,13 @@ template <typename T> struct SlotTable {
 static_assert(sizeof(SlotTable<double>) + 64 <= 32764, "batch parameter table exceeds the kernel parameter limit");
 
 // First statement of a kernel of a step's chain (scphd_filter.cu, chained): the kernel waits for
-// the end of the one before it; an ordinary launch passes at once.  In a batch the next kernel
-// may take the slots this one's last blocks leave free (64 filters of 256 parents: 2.43 -> 2.36
-// ms per step); a single filter's next kernel starts when this one's blocks have ended, since
-// waiting blocks would keep other filters' kernels from those slots (three filters of 1024
-// parents side by side: 291 us per step, 310 with early blocks, 289 so).
-template <bool kBatch = false> __device__ __forceinline__ void chain_wait() {
-    if (kBatch) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// the end of the one before it; an ordinary launch passes at once.  No kernel lets the next one
+// take the slots that its last blocks leave free: the waiting blocks keep other streams' kernels
+// from them (three filters of 1024 parents side by side: 291 us per step, 310 with early blocks;
+// a batch of eight filters of 256 parents beside a filter of 1024: 637 us for a step of both,
+// 701 with early blocks) and a small batch's own (373 us alone, 402), and gain a large batch
+// under half a percent (64 filters of 256 parents: 2.47 ms, 2.46 with early blocks).
+__device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
 template <typename T, int K, int PC = 0>
 __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
     k_cloud_fit_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int split) {
-    chain_wait<true>();
+    chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_fit[];
     const int q = blockIdx.x / split;
     const int2 fp = map[q];
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(__grid_constant__ const P
 template <typename T, int K>
 __global__ void __launch_bounds__(kPrepThreads)
     k_prep_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map) {
-    chain_wait<true>();
+    chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_prep[];
     const int2 fp = map[blockIdx.x];
     prep_body<T, K>(tab.prm[fp.x], tab.b[fp.x], fas[fp.x].cur, fp.y, reinterpret_cast<T*>(dsm_prep));
@@ -1093,7 +1093,7 @@ __global__ void __launch_bounds__(kLikThreads<T>) k_likelihood(__grid_constant__
 template <typename T, int K>
 __global__ void __launch_bounds__(kLikThreads<T>)
     k_likelihood_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int4* map) {
-    chain_wait<true>();
+    chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_lik[];
     const int4 e = map[blockIdx.x];
     const int M = fas[e.x].M;
@@ -2178,7 +2178,7 @@ template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
     k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int width,
                   int over) {
-    chain_wait<true>();
+    chain_wait();
     __shared__ int s_item;
     __shared__ unsigned s_listed;
     int2 fp = make_int2(0, 0);
@@ -2542,7 +2542,7 @@ __global__ void __launch_bounds__(1024)
 
 template <typename T>
 __global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas) {
-    chain_wait<true>();
+    chain_wait();
     const Bufs<T>& b = tab.b[blockIdx.x];
     const Params& prm = tab.prm[blockIdx.x];
     const FrameArgs& fa = fas[blockIdx.x];
@@ -2558,7 +2558,7 @@ __global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_co
 template <typename T>
 __global__ void k_predict_parents_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map,
                                         int* work) {
-    chain_wait<true>();
+    chain_wait();
     const int2 fp = map[blockIdx.x];
     const Bufs<T>& b = tab.b[fp.x];
     const FrameArgs& fa = fas[fp.x];
