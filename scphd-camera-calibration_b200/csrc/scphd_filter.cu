@@ -1444,6 +1444,10 @@ template <typename T> struct Batch final : scphd_batch {
     // captured after them.  Results do not depend on either.
     static constexpr int kPaths = 3, kTuneAfter = 16;
     const int merge_widths[kPaths] = {kMergeThreads, 128, 64};
+    // kernels set up in the slots of the running one (chain_wait): batches of 64 x 256 parents gain
+    // 3 % beside each other, ones of 6 x 1300 nothing, ones of 2048 to 4800 lose up to 6 %
+    static constexpr int kEarlyParents = 12000;
+    int early = 0;
     int path = 0;
     bool ripe = false;         // every member has seen kTuneAfter frames
     int fused_mode = 0;        // 1: the fused kernel instead
@@ -1503,6 +1507,7 @@ template <typename T> struct Batch final : scphd_batch {
         std::vector<std::vector<int4>> ml;
         stage_off.resize(F);
         for (int f = 0; f < F; ++f) lik_block = std::max(lik_block, likelihood_block<T>(fs[f]->prm.Mcap));
+        int parents = 0;
         for (int first = 0; first < F; first += kBatchSlots) {
             Group g;
             g.first = first;
@@ -1532,10 +1537,12 @@ template <typename T> struct Batch final : scphd_batch {
                 lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block));
             }
             g.n_parent = (int)mp.back().size();
+            parents += g.n_parent;
             g.n_pred = (int)mpred.back().size();
             g.n_lik = (int)ml.back().size();
             groups.push_back(g);
         }
+        early = parents >= kEarlyParents;
         Arena probe;
         probe.take<FrameArgs>(F);
         probe.take<double>(stage_total);
@@ -1625,7 +1632,7 @@ template <typename T> struct Batch final : scphd_batch {
         const bool timed = tuning && ripe && !capturing && pth < kPaths;
         for (const Group& g : groups) {
             chained(k_predict_parents_batch<T>, g.n_pred, 256, 0, stream, *g.tab, d_fa + g.first, g.map_pred,
-                                                                     pth == kPaths ? g.work : nullptr);
+                    pth == kPaths ? g.work : nullptr, early);
             LAUNCHED();
         }
         if (pth == kPaths) {
@@ -1640,10 +1647,11 @@ template <typename T> struct Batch final : scphd_batch {
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             for (const Group& g : groups) {
                 if (g.fit_p)
-                    chained(k_cloud_fit_batch<T, KK, kFitP>, g.n_parent * split, kFitThreads<T>, fit_smem, stream, *g.tab, d_fa + g.first, g.map_parent, split);
+                    chained(k_cloud_fit_batch<T, KK, kFitP>, g.n_parent * split, kFitThreads<T>, fit_smem, stream, *g.tab,
+                            d_fa + g.first, g.map_parent, split, early);
                 else
-                    chained(k_cloud_fit_batch<T, KK>, g.n_parent * split, kFitThreads<T>, fit_smem, stream, *g.tab, d_fa + g.first,
-                                                                                            g.map_parent, split);
+                    chained(k_cloud_fit_batch<T, KK>, g.n_parent * split, kFitThreads<T>, fit_smem, stream, *g.tab,
+                            d_fa + g.first, g.map_parent, split, early);
                 LAUNCHED();
             }
             if (fit_timed) {
@@ -1652,23 +1660,24 @@ template <typename T> struct Batch final : scphd_batch {
             }
             for (const Group& g : groups) {
                 chained(k_prep_batch<T, KK>, g.n_parent, kPrepThreads, prep_smem_bytes<T>(), stream, *g.tab, d_fa + g.first,
-                                                                                                   g.map_parent);
+                        g.map_parent, early);
                 LAUNCHED();
             }
             for (const Group& g : groups) {
-                chained(k_likelihood_batch<T, KK>, g.n_lik, lik_block, lik_smem, stream, *g.tab, d_fa + g.first, g.map_lik);
+                chained(k_likelihood_batch<T, KK>, g.n_lik, lik_block, lik_smem, stream, *g.tab, d_fa + g.first, g.map_lik,
+                        early);
                 LAUNCHED();
             }
             if (timed) CUDA_TRY(cudaEventRecord(tune_ev[0], stream));
             for (const Group& g : groups) {
                 chained(k_merge_batch<T, KK>, g.n_parent, merge_widths[pth], g.merge_first_smem[pth], stream, *g.tab,
-                        d_fa + g.first, g.map_parent, g.count, pth, 0);
+                        d_fa + g.first, g.map_parent, g.count, pth, 0, early);
                 LAUNCHED();
             }
             for (const Group& g : groups) {
                 if (!g.merge_over[pth]) continue;
                 chained(k_merge_batch<T, KK>, g.merge_over[pth], kMergeThreads, merge_smem, stream, *g.tab, d_fa + g.first,
-                        g.map_parent, g.count, pth, 1);
+                        g.map_parent, g.count, pth, 1, early);
                 LAUNCHED();
             }
             if (timed) {
@@ -1677,7 +1686,7 @@ template <typename T> struct Batch final : scphd_batch {
             }
         }
         for (const Group& g : groups) {
-            chained(k_weights_resample_batch<T>, g.count, 1024, 0, stream, *g.tab, d_fa + g.first);
+            chained(k_weights_resample_batch<T>, g.count, 1024, 0, stream, *g.tab, d_fa + g.first, early);
             LAUNCHED();
         }
         return SCPHD_OK;

@@ -105,13 +105,14 @@ template <typename T> struct SlotTable {
 static_assert(sizeof(SlotTable<double>) + 64 <= 32764, "batch parameter table exceeds the kernel parameter limit");
 
 // First statement of a kernel of a step's chain (scphd_filter.cu, chained): the kernel waits for
-// the end of the one before it; an ordinary launch passes at once.  No kernel lets the next one
-// take the slots that its last blocks leave free: the waiting blocks keep other streams' kernels
-// from them (three filters of 1024 parents side by side: 291 us per step, 310 with early blocks;
-// a batch of eight filters of 256 parents beside a filter of 1024: 637 us for a step of both,
-// 701 with early blocks) and a small batch's own (373 us alone, 402), and gain a large batch
-// under half a percent (64 filters of 256 parents: 2.47 ms, 2.46 with early blocks).
-__device__ __forceinline__ void chain_wait() {
+// the end of the one before it; an ordinary launch passes at once.  early: the next kernel may
+// take the slots that this one's last blocks leave free.  Its waiting blocks keep other streams'
+// kernels, and in a small batch this one's own, out of them: three filters of 1024 parents side
+// by side 291 us per step, 310 with early blocks; eight filters of 256 in a batch 361 us, 372;
+// that batch beside a filter of 1024 parents 640 us, 678.  Two batches of 64 filters of 256
+// parents stepped in turn gain: 2.42 ms, 2.34 with early blocks.
+__device__ __forceinline__ void chain_wait(int early = 0) {
+    if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
@@ -659,8 +660,8 @@ __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
 
 template <typename T, int K, int PC = 0>
 __global__ void __launch_bounds__(kFitThreads<T>, kFitBlocks<T>)
-    k_cloud_fit_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int split) {
-    chain_wait();
+    k_cloud_fit_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int split, int early) {
+    chain_wait(early);
     extern __shared__ __align__(16) unsigned char dsm_fit[];
     const int q = blockIdx.x / split;
     const int2 fp = map[q];
@@ -766,8 +767,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(__grid_constant__ const P
 
 template <typename T, int K>
 __global__ void __launch_bounds__(kPrepThreads)
-    k_prep_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map) {
-    chain_wait();
+    k_prep_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int early) {
+    chain_wait(early);
     extern __shared__ __align__(16) unsigned char dsm_prep[];
     const int2 fp = map[blockIdx.x];
     prep_body<T, K>(tab.prm[fp.x], tab.b[fp.x], fas[fp.x].cur, fp.y, reinterpret_cast<T*>(dsm_prep));
@@ -1092,8 +1093,8 @@ __global__ void __launch_bounds__(kLikThreads<T>) k_likelihood(__grid_constant__
 // map entry: (filter, parent, measurement block); blocks past a filter's M exit
 template <typename T, int K>
 __global__ void __launch_bounds__(kLikThreads<T>)
-    k_likelihood_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int4* map) {
-    chain_wait();
+    k_likelihood_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int4* map, int early) {
+    chain_wait(early);
     extern __shared__ __align__(16) unsigned char dsm_lik[];
     const int4 e = map[blockIdx.x];
     const int M = fas[e.x].M;
@@ -2177,8 +2178,8 @@ __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
 template <typename T, int K>
 __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
     k_merge_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map, int count, int width,
-                  int over) {
-    chain_wait();
+                  int over, int early) {
+    chain_wait(early);
     __shared__ int s_item;
     __shared__ unsigned s_listed;
     int2 fp = make_int2(0, 0);
@@ -2541,8 +2542,8 @@ __global__ void __launch_bounds__(1024)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas) {
-    chain_wait();
+__global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, int early) {
+    chain_wait(early);
     const Bufs<T>& b = tab.b[blockIdx.x];
     const Params& prm = tab.prm[blockIdx.x];
     const FrameArgs& fa = fas[blockIdx.x];
@@ -2557,8 +2558,8 @@ __global__ void __launch_bounds__(1024) k_weights_resample_batch(const __grid_co
 // counter (may be null).
 template <typename T>
 __global__ void k_predict_parents_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int2* map,
-                                        int* work) {
-    chain_wait();
+                                        int* work, int early) {
+    chain_wait(early);
     const int2 fp = map[blockIdx.x];
     const Bufs<T>& b = tab.b[fp.x];
     const FrameArgs& fa = fas[fp.x];
