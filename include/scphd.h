@@ -291,9 +291,10 @@ scphd_status scphd_device_bytes(const scphd_config* cfg, int64_t* bytes);
  * precision and meas_dim; they may differ in size.  While in a batch, the filters
  * issue all their work on the batch's stream (their own stream is restored by
  * scphd_batch_destroy), so single-filter calls stay ordered with batched steps.  With
- * use_graph != 0 the step is captured into a CUDA graph once its launch shapes are tuned
- * (on maps that have grown: after 16 frames of every member and six timed steps), and
- * later steps replay it.  A batched step gives each filter the same result as predict + update +
+ * use_graph != 0 the third step is captured into a CUDA graph and later steps replay it.
+ * The launch shapes are tuned on six steps (not replayed) once members with half of the
+ * parents have seen 16 frames; the graph is captured again after them.  Members keep the
+ * shapes, and trials not finished, for the next batch they are put in.  A batched step gives each filter the same result as predict + update +
  * resample on that filter alone.  This batching has no counterpart in the reference
  * (which runs one filter per process). */
 typedef struct scphd_frame {
@@ -326,9 +327,9 @@ void* scphd_batch_stream(scphd_batch* b);
 scphd_status scphd_batch_set_fused(scphd_batch* b, int32_t mode);
 scphd_status scphd_batch_get_fused(scphd_batch* b, int32_t* fused);
 /* The batch's cloud-fit tiling, as scphd_set_fit_split / scphd_get_fit_split (one
- * split for all member filters, tuned with the merge's block width on six steps once
- * every member has seen 16 frames, before the batch's graph is captured; set it before
- * the capture). */
+ * split for all member filters, tuned with the merge's block width; refused, like
+ * scphd_batch_set_fused, once a graph is captured and all members have been stepped
+ * seven times after their 16th frame). */
 scphd_status scphd_batch_set_fit_split(scphd_batch* b, int32_t blocks_per_parent);
 scphd_status scphd_batch_get_fit_split(scphd_batch* b, int32_t* blocks_per_parent, int32_t* tuned);
 

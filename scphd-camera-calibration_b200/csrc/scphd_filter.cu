@@ -97,6 +97,18 @@ __attribute__((visibility("hidden"))) scphd_status scphd_fail_internal(scphd_sta
     return fail(st, msg);
 }
 
+// A batch's launch shapes and how far it is with timing them (Batch::tune).  Members keep a copy
+// when their batch goes, so that the next one, which a server makes whenever a job arrives or
+// retires, goes on from it.  Times are per parent, in ms.
+struct BatchTune {
+    uint64_t id = 0;       // of the batch that began it (0: none)
+    int parents = 0;       // that batch's
+    bool width_open = true, split_open = true;   // still to be timed
+    int width = 0, split = 0;                    // the choice, or what is used until there is one
+    int width_trials = 0, split_trials = 0;
+    double width_ms[3] = {0, 0, 0}, split_ms[3] = {0, 0, 0};
+};
+
 struct scphd_filter {
     scphd_config cfg;
     Params prm;
@@ -157,6 +169,7 @@ struct scphd_filter {
     int merge_trials = 0, merge_pending = -1, merge_chosen = -1;
     double merge_ms[kMergeWidths] = {0, 0, 0};
     cudaEvent_t merge_ev[2] = {nullptr, nullptr};
+    BatchTune batch_tune;   // of the batch that last held this filter
     int merge_width() const { return merge_chosen >= 0 ? merge_chosen : (shapes[chosen].merge_threads == kMergeThreads ? 0 : 1); }
     // whether the next update takes the fused path (profiling times the stage kernels
     // one by one)
@@ -1437,42 +1450,48 @@ template <typename T> struct Batch final : scphd_batch {
     size_t lik_smem = 0;
     int lik_block = 32;
     // the update path: the stage kernels with 256, 128 or 64 threads per merge block, or the
-    // fused kernel when requested (scphd_batch_set_fused).  The width is tuned by the merge
-    // launches' own time, twice each, with the cloud fit's split below, on the first six steps
-    // whose members have all seen kTuneAfter frames (their maps have grown: at 64 filters of 256
-    // parents the first frames' maps chose 256 threads, 64 are 1.2 times as fast); the graph is
-    // captured after them.  Results do not depend on either.
-    static constexpr int kPaths = 3, kTuneAfter = 16;
+    // fused kernel when requested (scphd_batch_set_fused).  The merge width is timed by the merge
+    // launches, the cloud fit's blocks per parent (1, 2, 4) by its own, each shape twice, on the
+    // first steps on which members with half of the parents have seen kTuneAfter frames (their
+    // maps have grown: at 64 filters of 256 parents the first frames' maps chose 256 threads, 64
+    // are 1.2 times as fast).  A batch of which members with half of the parents come from one
+    // batch of at most twice or at least half its parents goes on with that one's choice or
+    // trials.  Results do not depend on either.
+    static constexpr int kPaths = 3, kFitSplits = 3, kTuneAfter = 16;
     const int merge_widths[kPaths] = {kMergeThreads, 128, 64};
+    const int fit_splits[kFitSplits] = {1, 2, 4};
+    BatchTune tune;
+    int fixed_split = -1;      // scphd_batch_set_fit_split's (index), -1: none
+    int parents = 0;
+    bool ripe = false;         // members with half of the parents have seen kTuneAfter frames
+    int grown_steps = 0;       // steps on which all of them had
     // kernels set up in the slots of the running one (chain_wait): batches of 64 x 256 parents gain
     // 3 % beside each other, ones of 6 x 1300 nothing, ones of 2048 to 4800 lose up to 6 %
     static constexpr int kEarlyParents = 12000;
     int early = 0;
-    int path = 0;
-    bool ripe = false;         // every member has seen kTuneAfter frames
     int fused_mode = 0;        // 1: the fused kernel instead
     size_t fused_smem = 0;
     int fused_grid = 0;        // 0: the fused kernel is unavailable
-    bool tuning = true;
-    bool capturing = false;
-    int tune_trials = 0, tune_pending = -1;
-    double tune_ms[kPaths] = {0, 0, 0};
-    int path_now() const {     // the path of the step being enqueued (kPaths: fused)
-        if (fused_mode == 1 && fused_grid > 0) return kPaths;
-        return (tuning && ripe && !capturing) ? tune_trials % kPaths : path;
-    }
+    bool fused_now() const { return fused_mode == 1 && fused_grid > 0; }
+    bool width_timed() const { return tune.width_open && ripe && !fused_now(); }
+    bool split_timed() const { return tune.split_open && ripe && !fused_now() && fixed_split < 0; }
+    // of the step being enqueued (path kPaths: fused)
+    int path_now() const { return fused_now() ? kPaths : (width_timed() ? tune.width_trials % kPaths : tune.width); }
+    int split_now() const { return fixed_split >= 0 ? fixed_split : (split_timed() ? tune.split_trials % kFitSplits : tune.split); }
+    // steps before a capture: for a batch that lives for a step or two (a server's, between two
+    // arrivals) it does not pay
+    static constexpr int kGraphAfter = 2;
+    int steps = 0;
+    int width_pending = -1, split_pending = -1;
     cudaEvent_t tune_ev[2] = {nullptr, nullptr};
-    // blocks per parent of the cloud fit (1, 2, 4), tuned by the cloud-fit launches' own time
-    static constexpr int kFitSplits = 3;
-    const int fit_splits[kFitSplits] = {1, 2, 4};
-    bool fit_tuning = true;
-    int fit_trials = 0, fit_pending = -1, fit_chosen = 0;
-    double fit_ms[kFitSplits] = {0, 0, 0};
     cudaEvent_t fit_ev[2] = {nullptr, nullptr};
     void* dev_mem = nullptr;
 
     ~Batch() override {
         if (stream) cudaStreamSynchronize(stream);
+        if (tune_collect() == SCPHD_OK)
+            for (scphd_filter* f : fs)
+                if (f->batch == this) f->batch_tune = tune;
         for (cudaEvent_t e : tune_ev)
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : fit_ev)
@@ -1507,7 +1526,6 @@ template <typename T> struct Batch final : scphd_batch {
         std::vector<std::vector<int4>> ml;
         stage_off.resize(F);
         for (int f = 0; f < F; ++f) lik_block = std::max(lik_block, likelihood_block<T>(fs[f]->prm.Mcap));
-        int parents = 0;
         for (int first = 0; first < F; first += kBatchSlots) {
             Group g;
             g.first = first;
@@ -1543,6 +1561,7 @@ template <typename T> struct Batch final : scphd_batch {
             groups.push_back(g);
         }
         early = parents >= kEarlyParents;
+        adopt_tune();
         Arena probe;
         probe.take<FrameArgs>(F);
         probe.take<double>(stage_total);
@@ -1626,10 +1645,34 @@ template <typename T> struct Batch final : scphd_batch {
         return SCPHD_OK;
     }
 
+    // the tuning of the batch that most of the members' parents were last in
+    void adopt_tune() {
+        static std::atomic<uint64_t> next_id{1};
+        const BatchTune* most = nullptr;
+        long long most_parents = 0;
+        for (const scphd_filter* f : fs) {
+            if (!f->batch_tune.id) continue;
+            long long n = 0;
+            for (const scphd_filter* o : fs) n += o->batch_tune.id == f->batch_tune.id ? o->prm.N : 0;
+            if (n > most_parents) {
+                most_parents = n;
+                most = &f->batch_tune;
+            }
+        }
+        if (most && 2 * most_parents >= parents && parents <= 2 * most->parents && most->parents <= 2 * parents) {
+            tune = *most;
+            return;
+        }
+        tune = BatchTune();
+        tune.id = next_id.fetch_add(1);
+        tune.parents = parents;
+        if (most) tune.width = most->width, tune.split = most->split;   // until its own are timed
+    }
+
     // kernels of one frame, stage by stage over the groups
     template <int KK> scphd_status launch_all() {
         const int pth = path_now();
-        const bool timed = tuning && ripe && !capturing && pth < kPaths;
+        const bool timed = width_timed();
         for (const Group& g : groups) {
             chained(k_predict_parents_batch<T>, g.n_pred, 256, 0, stream, *g.tab, d_fa + g.first, g.map_pred,
                     pth == kPaths ? g.work : nullptr, early);
@@ -1642,8 +1685,8 @@ template <typename T> struct Batch final : scphd_batch {
                 LAUNCHED();
             }
         } else {
-            const bool fit_timed = fit_tuning && ripe && !capturing;
-            const int fsi = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fsi];
+            const bool fit_timed = split_timed();
+            const int fsi = split_now(), split = fit_splits[fsi];
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             for (const Group& g : groups) {
                 if (g.fit_p)
@@ -1656,7 +1699,7 @@ template <typename T> struct Batch final : scphd_batch {
             }
             if (fit_timed) {
                 CUDA_TRY(cudaEventRecord(fit_ev[1], stream));
-                fit_pending = fsi;
+                split_pending = fsi;
             }
             for (const Group& g : groups) {
                 chained(k_prep_batch<T, KK>, g.n_parent, kPrepThreads, prep_smem_bytes<T>(), stream, *g.tab, d_fa + g.first,
@@ -1682,7 +1725,7 @@ template <typename T> struct Batch final : scphd_batch {
             }
             if (timed) {
                 CUDA_TRY(cudaEventRecord(tune_ev[1], stream));
-                tune_pending = pth;
+                width_pending = pth;
             }
         }
         for (const Group& g : groups) {
@@ -1699,57 +1742,61 @@ template <typename T> struct Batch final : scphd_batch {
         return n;
     }
 
+    // the graph of a batch that has still to time its shapes, or was made of grown members less
+    // than its trials' steps ago, gives way to other settings
+    bool closed() const { return captured && (fused_now() || grown_steps > 2 * kPaths); }
+    scphd_status drop_graph() {
+        if (!captured) return SCPHD_OK;
+        CUDA_TRY(cudaStreamSynchronize(stream));   // it may still run
+        CUDA_TRY(cudaGraphExecDestroy(exec));
+        exec = nullptr;
+        captured = false;
+        return SCPHD_OK;
+    }
+
     scphd_status set_fused(int mode) override {
         if (mode < 0 || mode > 1) return fail(SCPHD_ERR_INVALID, "mode must be 0 or 1");
         if (mode == 1 && fused_grid <= 0)
             return fail(SCPHD_ERR_CAPACITY, "the fused kernel needs more shared memory than a block has");
-        if (captured) return fail(SCPHD_ERR_INVALID, "the batch's step graph is already captured");
+        if (closed()) return fail(SCPHD_ERR_INVALID, "the batch's step graph is already captured");
         fused_mode = mode;
-        if (mode == 1) tuning = fit_tuning = false;   // the stage kernels' shapes are not needed
-        return SCPHD_OK;
+        return drop_graph();
     }
     int fused_path() const override { return path_now() == kPaths ? 1 : 0; }
     scphd_status set_fit_split(int blocks_per_parent) override {
-        if (captured) return fail(SCPHD_ERR_INVALID, "the batch's step graph is already captured");
+        if (closed()) return fail(SCPHD_ERR_INVALID, "the batch's step graph is already captured");
         for (int k = 0; k < kFitSplits; ++k)
             if (fit_splits[k] == blocks_per_parent) {
-                fit_tuning = false;
-                fit_pending = -1;
-                fit_chosen = k;
-                return SCPHD_OK;
+                fixed_split = k;
+                return drop_graph();
             }
         return fail(SCPHD_ERR_INVALID, "blocks_per_parent must be 1, 2 or 4");
     }
     void get_fit_split(int32_t* blocks_per_parent, int32_t* tuned) const override {
-        if (blocks_per_parent) *blocks_per_parent = fit_splits[fit_chosen];
-        if (tuned) *tuned = fit_tuning ? 0 : 1;
+        if (blocks_per_parent) *blocks_per_parent = fit_splits[fixed_split >= 0 ? fixed_split : tune.split];
+        if (tuned) *tuned = tune.split_open && fixed_split < 0 && !fused_now() ? 0 : 1;
     }
 
-    scphd_status tune_collect() {
-        if (fit_pending >= 0) {
-            CUDA_TRY(cudaEventSynchronize(fit_ev[1]));
-            float ms = 0;
-            CUDA_TRY(cudaEventElapsedTime(&ms, fit_ev[0], fit_ev[1]));
-            fit_ms[fit_pending] += ms;
-            fit_pending = -1;
-            if (++fit_trials >= 2 * kFitSplits) {
-                fit_tuning = false;
-                for (int k = 1; k < kFitSplits; ++k)
-                    if (fit_ms[k] < fit_ms[fit_chosen]) fit_chosen = k;
-            }
-        }
-        if (tune_pending < 0) return SCPHD_OK;
-        CUDA_TRY(cudaEventSynchronize(tune_ev[1]));
-        float ms = 0;
-        CUDA_TRY(cudaEventElapsedTime(&ms, tune_ev[0], tune_ev[1]));
-        tune_ms[tune_pending] += ms;
-        tune_pending = -1;
-        if (++tune_trials >= 2 * kPaths) {
-            tuning = false;
-            for (int k = 1; k < kPaths; ++k)
-                if (tune_ms[k] < tune_ms[path]) path = k;
+    // the last step's trial: the shape's time; after two of each the fastest is kept
+    static scphd_status collect(const cudaEvent_t ev[2], int& pending, int parents, int shapes, bool& open, int& chosen,
+                                int& trials, double* ms) {
+        if (pending < 0) return SCPHD_OK;
+        float t = 0;
+        CUDA_TRY(cudaEventSynchronize(ev[1]));
+        CUDA_TRY(cudaEventElapsedTime(&t, ev[0], ev[1]));
+        ms[pending] += t / parents;
+        pending = -1;
+        if (++trials >= 2 * shapes) {
+            open = false;
+            chosen = (int)(std::min_element(ms, ms + shapes) - ms);
         }
         return SCPHD_OK;
+    }
+    scphd_status tune_collect() {
+        const scphd_status s =
+            collect(fit_ev, split_pending, parents, kFitSplits, tune.split_open, tune.split, tune.split_trials, tune.split_ms);
+        if (s != SCPHD_OK) return s;
+        return collect(tune_ev, width_pending, parents, kPaths, tune.width_open, tune.width, tune.width_trials, tune.width_ms);
     }
 
     // the step's measurements and frame arguments to the device, ahead of its kernels on
@@ -1818,21 +1865,24 @@ template <typename T> struct Batch final : scphd_batch {
             const scphd_status ts = tune_collect();
             if (ts != SCPHD_OK) return ts;
         }
-        if (!ripe) {
-            ripe = true;
-            for (int f = 0; f < F; ++f) ripe = ripe && filt(f)->frame > kTuneAfter;
-        }
+        int grown = 0;
+        for (int f = 0; f < F; ++f) grown += filt(f)->frame > kTuneAfter ? fs[f]->prm.N : 0;
+        ripe = 2 * grown >= parents;
+        grown_steps += grown == parents;
         {
             const scphd_status cs = copy_in();
             if (cs != SCPHD_OK) return cs;
         }
-        if (use_graph && !tuning && !fit_tuning) {
+        const bool timing = width_timed() || split_timed();
+        if (timing) {   // the shapes change
+            const scphd_status ds = drop_graph();
+            if (ds != SCPHD_OK) return ds;
+        }
+        if (use_graph && !timing && (captured || fused_now() || steps >= kGraphAfter)) {
             if (!captured) {
                 cudaGraph_t g = nullptr;
                 CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-                capturing = true;
                 scphd_status s = enqueue();
-                capturing = false;
                 cudaError_t e = cudaStreamEndCapture(stream, &g);
                 if (s != SCPHD_OK) return s;
                 if (e != cudaSuccess) return fail(SCPHD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -1849,6 +1899,7 @@ template <typename T> struct Batch final : scphd_batch {
             scphd_status s = enqueue();
             if (s != SCPHD_OK) return s;
         }
+        ++steps;
         for (int f = 0; f < F; ++f) {
             Filter<T>* fl = filt(f);
             fl->cur ^= 1;

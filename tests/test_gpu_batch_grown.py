@@ -101,3 +101,81 @@ def test_resident_batch_takes_one_merge_launch(pkg, precision):
         assert pkg.kernel_launches() - before == 6
     assert_same(alone, batched, "last")
     batch.close()
+
+
+def _step_all(pkg, ms, alone, batch, k):
+    fr = frames(ms, k, 3)
+    for f, (u, v, d, fixed) in zip(alone, fr):
+        f.step(pkg.scene.DT, u, v, fixed_camera=fixed, d=d)
+    batch.step(pkg.scene.DT, fr)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_rebuilt_batch_goes_on_with_its_members_shapes(pkg, precision):
+    """Batches made anew from the same filters, as a server makes them: trials are carried on, a
+    choice is kept, and a young member neither holds back nor spoils the others."""
+    ms = members(pkg, precision, 3, 30)
+    alone = [pkg.SCPHDCameraCalibration(c) for _, c, _ in ms]
+    batched = [pkg.SCPHDCameraCalibration(c) for _, c, _ in ms]
+    batch = pkg.SCPHDBatch(batched[:2], use_graph=True)
+    for k in range(18):   # 16 frames, two of the six trials
+        _step_all(pkg, ms[:2], alone[:2], batch, k)
+    assert not batch.fit_split()["fit_tuned"]
+    batch.set_fit_split(2)   # open until the shapes are settled: the graph of the first steps goes
+    _step_all(pkg, ms[:2], alone[:2], batch, 18)
+    batch.close()
+    batch = pkg.SCPHDBatch(batched, use_graph=True)   # with a young third member of fewer parents
+    tuned = []
+    for k in range(19, 26):
+        _step_all(pkg, ms, alone, batch, k)
+        tuned.append(batch.fit_split()["fit_tuned"])
+    assert tuned == [False] * 4 + [True] * 3   # four more trials, seen on the step after them
+    split = batch.fit_split()
+    batch.close()
+    batch = pkg.SCPHDBatch(batched, use_graph=True)
+    assert batch.fit_split() == split
+    for k in range(26, 31):
+        _step_all(pkg, ms, alone, batch, k)
+    assert_same(alone, batched, "rebuilt")
+    batch.close()
+
+
+def test_settled_batch_refuses_other_shapes(pkg):
+    ms = members(pkg, 0, 3, 30)[:2]
+    alone = [pkg.SCPHDCameraCalibration(c) for _, c, _ in ms]
+    batched = [pkg.SCPHDCameraCalibration(c) for _, c, _ in ms]
+    batch = pkg.SCPHDBatch(batched, use_graph=True)
+    for k in range(24):
+        _step_all(pkg, ms, alone, batch, k)
+    with pytest.raises(pkg.ScphdError):
+        batch.set_fit_split(4)
+    with pytest.raises(pkg.ScphdError):
+        batch.set_fused(1)
+    batch.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_served_long_jobs_equal_jobs_alone(pkg, precision):
+    """Jobs that outlive the tuning, with others arriving and retiring beside them."""
+    S = pkg.scene
+    jobs = []
+    for i, (n, nf) in enumerate([(96, 40), (64, 33), (40, 9), (30, 12), (50, 27)]):
+        sc = S.make_scene(n_landmarks=12 + 2 * i, n_frames=nf, clutter_rate=4.0, seed=S.scene_seed(4, 30 + i))
+        jobs.append((sc, S.filter_config(n, 96, 64, 4.0, precision=precision, calib=sc.calib, seed=800 + i,
+                                         particles_per_feature=36 + 8 * i)))
+    srv = pkg.SCPHDServer(int(2e9), precision=precision, meas_dim=3, use_graph=True)
+    arrive = {0: [0, 1], 5: [2], 19: [3], 25: [4]}
+    ids = {}
+    for it in range(60):
+        for i in arrive.get(it, []):
+            ids[i] = srv.submit(jobs[i][1], jobs[i][0].frames, jobs[i][0].fixed, S.DT)
+        srv.step()
+    srv.drain()
+    assert srv.stats()["done"] == len(jobs) and srv.stats()["rebuilds"] >= 5
+    for i, (sc, cfg) in enumerate(jobs):
+        f = pkg.SCPHDCameraCalibration(cfg)
+        for k, z in enumerate(sc.frames):
+            f.step(S.DT, z[:, 0], z[:, 1], fixed_camera=sc.fixed[k], d=z[:, 2])
+        for x, y in zip(srv.result(ids[i]), f.particles()):
+            assert np.array_equal(x, y), f"job {i}"
+    srv.close()
