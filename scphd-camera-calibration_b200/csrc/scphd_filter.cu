@@ -311,11 +311,17 @@ public:
     void* arena_ptr = nullptr;
     double* dump = nullptr;   // Gcap x 7 x P: a parent's cloud for the host
     double* ell_out = nullptr;   // N x Mcap: the normalisers for the host
-    // Results of up to kReadBytes come back through page-locked memory behind h_stage: the copies
-    // are queued and waited for once, where each copy to a caller's pageable array waits for
-    // itself (24 KB of parents' states and weights 36 -> 15 us)
+    // Results of up to kReadBytes come back through page-locked memory: the copies are queued and
+    // waited for once, where each copy to a caller's pageable array waits for itself (24 KB of
+    // parents' states and weights 36 -> 15 us).  The parents' rows have theirs behind h_stage;
+    // for larger results (normalisers, a map's clouds) the filter's largest is page-locked when
+    // the first is read, so that the many filters of a batch or a server, which are not read
+    // that way, do not hold 512 KB each.
     static constexpr size_t kReadBytes = 512 * 1024;
     char* h_read = nullptr;
+    char* h_large = nullptr;
+    size_t read_bytes = 0, large_bytes = 0;
+    static size_t padded(size_t bytes) { return (bytes + 15) & ~(size_t)15; }
     struct Piece {
         void* to;
         const void* from;
@@ -323,20 +329,22 @@ public:
     };
     scphd_status fetch(std::initializer_list<Piece> pieces) {
         size_t total = 0;
-        for (const Piece& q : pieces) total += (q.bytes + 15) & ~(size_t)15;
-        const bool staged = total <= kReadBytes;
-        char* at = h_read;
+        for (const Piece& q : pieces) total += padded(q.bytes);
+        const bool staged = total <= std::max(read_bytes, large_bytes);
+        if (staged && total > read_bytes && !h_large) CUDA_TRY(cudaMallocHost(&h_large, large_bytes));
+        char* const room = total <= read_bytes ? h_read : h_large;
+        char* at = room;
         for (const Piece& q : pieces) {
             if (!q.to || !q.bytes) continue;
             CUDA_TRY(cudaMemcpyAsync(staged ? at : q.to, q.from, q.bytes, cudaMemcpyDeviceToHost, stream));
-            at += (q.bytes + 15) & ~(size_t)15;
+            at += padded(q.bytes);
         }
         CUDA_TRY(cudaStreamSynchronize(stream));
-        at = h_read;
+        at = room;
         for (const Piece& q : pieces) {
             if (!staged || !q.to || !q.bytes) continue;
             std::memcpy(q.to, at, q.bytes);
-            at += (q.bytes + 15) & ~(size_t)15;
+            at += padded(q.bytes);
         }
         return SCPHD_OK;
     }
@@ -349,6 +357,7 @@ public:
         if (stream) cudaStreamSynchronize(stream);
         if (arena_ptr) cudaFree(arena_ptr);
         if (h_stage) cudaFreeHost(h_stage);
+        if (h_large) cudaFreeHost(h_large);
         if (stage_ev) cudaEventDestroy(stage_ev);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -403,7 +412,12 @@ public:
         CUDA_TRY(cudaEventCreate(&merge_ev[1]));
         CUDA_TRY(cudaEventCreateWithFlags(&stage_ev, cudaEventDisableTiming));
         const size_t stage_bytes = (sizeof(double) * 3 * prm.Mcap + 255) & ~(size_t)255;
-        CUDA_TRY(cudaMallocHost(&h_stage, stage_bytes + kReadBytes));
+        const size_t parents = prm.N, gaussians = prm.Gcap;
+        read_bytes = std::min(kReadBytes, std::max<size_t>(256, padded(96 * parents) + padded(8 * parents)));
+        large_bytes = std::min(kReadBytes, std::max({padded(8 * parents * prm.Mcap) + padded(8 * parents),
+                                                     padded(48 * gaussians * prm.P) + padded(8 * gaussians * prm.P),
+                                                     padded(sizeof(T) * gaussians * kRow)}));
+        CUDA_TRY(cudaMallocHost(&h_stage, stage_bytes + read_bytes));
         h_read = reinterpret_cast<char*>(h_stage) + stage_bytes;
         Arena probe;
         carve(probe);
