@@ -448,13 +448,15 @@ public:
             CUDA_TRY(allow_dynamic_smem((const void*)k_merge<T, 2>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit<T, 2>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit<T, 2, kFitP>));
-            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 2>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 2, 1>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 2, kLikPerMost<T>>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_prep<T, 2>));
         } else {
             CUDA_TRY(allow_dynamic_smem((const void*)k_merge<T, 3>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit<T, 3>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit<T, 3, kFitP>));
-            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 3>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 3, 1>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood<T, 3, kLikPerMost<T>>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_prep<T, 3>));
         }
         {
@@ -575,10 +577,12 @@ public:
             LAUNCHED();
             stage_end(h);
             if (M > 0) {
-                const int bs = sh.lik_full ? likelihood_block<T>(M) : 128 / kLikPer<T>, per = bs * kLikPer<T>;
-                dim3 grid(N, (M + per - 1) / per);
+                const int per = likelihood_per<T>(N, M), bs = sh.lik_full ? likelihood_block(M, per) : 128 / per;
+                const dim3 grid(N, (M + bs * per - 1) / (bs * per));
+                const size_t smem = likelihood_smem_bytes<T>(prm.Gcap, bs, per);
                 h = stage_begin(2);
-                chained(k_likelihood<T, K>, grid, bs, likelihood_smem_bytes<T>(prm.Gcap, bs), stream, prm, b, cur, M);
+                if (per == 1) chained(k_likelihood<T, K, 1>, grid, bs, smem, stream, prm, b, cur, M);
+                else chained(k_likelihood<T, K, kLikPerMost<T>>, grid, bs, smem, stream, prm, b, cur, M);
                 LAUNCHED();
                 stage_end(h);
             }
@@ -1462,7 +1466,7 @@ template <typename T> struct Batch final : scphd_batch {
     size_t merge_need = 0;       // the limit's (merge_limit_bytes)
     size_t fit_smem = 0;
     size_t lik_smem = 0;
-    int lik_block = 32;
+    int lik_block = 32, lik_per = 1;   // the likelihood's threads per block, measurements per thread
     // the update path: the stage kernels with 256, 128 or 64 threads per merge block, or the
     // fused kernel when requested (scphd_batch_set_fused).  The merge width is timed by the merge
     // launches, the cloud fit's blocks per parent (1, 2, 4) by its own, each shape twice, on the
@@ -1476,7 +1480,7 @@ template <typename T> struct Batch final : scphd_batch {
     const int fit_splits[kFitSplits] = {1, 2, 4};
     BatchTune tune;
     int fixed_split = -1;      // scphd_batch_set_fit_split's (index), -1: none
-    int parents = 0;
+    int parents = 0;           // of all members
     bool ripe = false;         // members with half of the parents have seen kTuneAfter frames
     int grown_steps = 0;       // steps on which all of them had
     // kernels set up in the slots of the running one (chain_wait): batches of 64 x 256 parents gain
@@ -1539,7 +1543,13 @@ template <typename T> struct Batch final : scphd_batch {
         std::vector<std::vector<int2>> mp, mpred;
         std::vector<std::vector<int4>> ml;
         stage_off.resize(F);
-        for (int f = 0; f < F; ++f) lik_block = std::max(lik_block, likelihood_block<T>(fs[f]->prm.Mcap));
+        int most = 0;
+        for (int f = 0; f < F; ++f) {
+            parents += fs[f]->prm.N;
+            most = std::max(most, fs[f]->prm.Mcap);
+        }
+        lik_per = likelihood_per<T>(parents, most);
+        lik_block = likelihood_block(most, lik_per);
         for (int first = 0; first < F; first += kBatchSlots) {
             Group g;
             g.first = first;
@@ -1557,7 +1567,7 @@ template <typename T> struct Batch final : scphd_batch {
                 g.tab->b[i] = fl->b;
                 for (int q = 0; q < pr.N; ++q) mp.back().push_back(make_int2(i, q));
                 for (int q = 0; q < pr.N; q += 256) mpred.back().push_back(make_int2(i, q));
-                const int per = lik_block * kLikPer<T>, mb = (pr.Mcap + per - 1) / per;
+                const int per = lik_block * lik_per, mb = (pr.Mcap + per - 1) / per;
                 for (int q = 0; q < pr.N; ++q)
                     for (int k = 0; k < mb; ++k) ml.back().push_back(make_int4(i, q, k, 0));
                 stage_off[first + i] = stage_total;
@@ -1566,10 +1576,9 @@ template <typename T> struct Batch final : scphd_batch {
                 merge_smem = std::max(merge_smem, merge_shared_bytes<T>(pr.Scap, pr.Gcap, kMergeThreads / 32));
                 fit_smem = std::max(fit_smem, fit_kernel_smem_bytes<T>(pr.P));
                 fused_smem = std::max(fused_smem, fused_smem_bytes<T>(pr.P, pr.Gcap, pr.Scap));
-                lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block));
+                lik_smem = std::max(lik_smem, likelihood_smem_bytes<T>(pr.Gcap, lik_block, lik_per));
             }
             g.n_parent = (int)mp.back().size();
-            parents += g.n_parent;
             g.n_pred = (int)mpred.back().size();
             g.n_lik = (int)ml.back().size();
             groups.push_back(g);
@@ -1620,13 +1629,15 @@ template <typename T> struct Batch final : scphd_batch {
             CUDA_TRY(allow_dynamic_smem((const void*)k_merge_batch<T, 2>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit_batch<T, 2>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit_batch<T, 2, kFitP>));
-            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 2>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 2, 1>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 2, kLikPerMost<T>>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_prep_batch<T, 2>));
         } else {
             CUDA_TRY(allow_dynamic_smem((const void*)k_merge_batch<T, 3>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit_batch<T, 3>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_cloud_fit_batch<T, 3, kFitP>));
-            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 3>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 3, 1>));
+            CUDA_TRY(allow_dynamic_smem((const void*)k_likelihood_batch<T, 3, kLikPerMost<T>>));
             CUDA_TRY(allow_dynamic_smem((const void*)k_prep_batch<T, 3>));
         }
         {
@@ -1721,8 +1732,12 @@ template <typename T> struct Batch final : scphd_batch {
                 LAUNCHED();
             }
             for (const Group& g : groups) {
-                chained(k_likelihood_batch<T, KK>, g.n_lik, lik_block, lik_smem, stream, *g.tab, d_fa + g.first, g.map_lik,
-                        early);
+                if (lik_per == 1)
+                    chained(k_likelihood_batch<T, KK, 1>, g.n_lik, lik_block, lik_smem, stream, *g.tab, d_fa + g.first,
+                            g.map_lik, early);
+                else
+                    chained(k_likelihood_batch<T, KK, kLikPerMost<T>>, g.n_lik, lik_block, lik_smem, stream, *g.tab,
+                            d_fa + g.first, g.map_lik, early);
                 LAUNCHED();
             }
             if (timed) CUDA_TRY(cudaEventRecord(tune_ev[0], stream));

@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kPrepThreads)
 // Normaliser ell_{p,m} = logsumexp_j(log w_{j,m}) (+) log(M w0 + kappa)
 // (.cu:1729-1768) and survivor compaction: w_{j,m} = exp(log w - ell) >= min_weight
 // with a PD posterior (updateKernel, kernels.cu:622-657), births likewise.
-// A thread per measurement, or per two in FP32; a block covers the frame's measurements
+// A thread per measurement, or per two in large FP32 launches (likelihood_per); a block covers the frame's measurements
 // (up to 1024, by a multiple of 32 threads; more take more blocks) and stages the
 // parent's Gaussian terms once in shared memory for both passes.  Since ell >= bpc =
 // log(M w0 + kappa) (the sum inside the log holds exp(0) = 1 around its larger term),
@@ -788,13 +788,21 @@ __global__ void __launch_bounds__(kPrepThreads)
 //
 // FP32 takes two Gaussians at a time in packed operations: their terms are staged side by
 // side, the measurement is doubled in registers, and the exponentials are summed one by one,
-// in the Gaussians' order (the one-by-one form's normalisers bit for bit); a thread has two
-// measurements, so that terms read from shared memory serve four pairs.  Per launch of 4096
-// parents x 256 Gaussians: 0.188 ms one by one, 0.175 in pairs, 0.169 with two measurements.
+// in the Gaussians' order (the one-by-one form's normalisers bit for bit); with two measurements
+// a thread, terms read from shared memory serve four pairs.  Per launch of 4096 parents x 256
+// Gaussians: 0.188 ms one by one, 0.175 in pairs, 0.169 with two measurements.
 // FP64 takes Gaussians and measurements one by one.
 constexpr int kLikCand = 15;   // candidate survivors remembered per measurement
-template <typename T> constexpr int kLikPer = sizeof(T) == 4 ? 2 : 1;          // measurements of a thread
-template <typename T> constexpr int kLikThreads = 1024 / kLikPer<T>;            // of a block, at most
+template <typename T> constexpr int kLikPerMost = sizeof(T) == 4 ? 2 : 1;   // measurements of a thread, at most
+// Measurements of a thread, for M of them and N parents in a launch.  Two halve a launch's warps,
+// which small launches miss, and leave lanes idle where M fills fewer whole warps' doubles:
+// at 1024 parents 1.03 to 1.27 times as long as with one (39 to 323 measurements), at 8192
+// 0.93 to 0.97 where at most a tenth more lanes are idle (39, 104, 169, 323 measurements), 1.09
+// and 1.15 at 68 and 86.
+template <typename T> inline int likelihood_per(int N, int M) {
+    return sizeof(T) == 4 && N >= 4000 && 10 * ((M + 63) / 64 * 64) <= 11 * ((M + 31) / 32 * 32) ? 2 : 1;
+}
+constexpr int kLikThreads = 1024;   // of a block, at most (with two measurements a thread: half)
 typedef unsigned short LikIndex;   // shared memory holds fewer than 2^16 Gaussians' terms
 // two Gaussians' log-constants, S^-1, negated means and pD flags, the even one's low; behind
 // the last Gaussian of an odd map its own terms again with log-constant -inf
@@ -803,13 +811,13 @@ constexpr int kLpA = 1, kLpMean = 7, kLpFlag = 10;
 template <typename T> __host__ __device__ inline int likelihood_rows(int Gcap) {
     return sizeof(T) == 4 ? (Gcap + 1) / 2 * 2 : Gcap;
 }
-template <typename T> __host__ __device__ inline size_t likelihood_smem_bytes(int Gcap, int block) {
-    return (size_t)likelihood_rows<T>(Gcap) * kLikTerms * sizeof(T) +
-           (size_t)block * kLikPer<T> * kLikCand * sizeof(LikIndex);
+// per: measurements of a thread
+template <typename T> __host__ __device__ inline size_t likelihood_smem_bytes(int Gcap, int block, int per) {
+    return (size_t)likelihood_rows<T>(Gcap) * kLikTerms * sizeof(T) + (size_t)block * per * kLikCand * sizeof(LikIndex);
 }
-template <typename T> __host__ __device__ inline int likelihood_block(int M) {
-    const int r = ((M + kLikPer<T> - 1) / kLikPer<T> + 31) / 32 * 32;
-    return r < 32 ? 32 : (r > kLikThreads<T> ? kLikThreads<T> : r);
+__host__ __device__ inline int likelihood_block(int M, int per) {
+    const int r = ((M + per - 1) / per + 31) / 32 * 32, most = kLikThreads / per;
+    return r < 32 ? 32 : (r > most ? most : r);
 }
 
 __device__ __forceinline__ void load_terms(const float* src, float* t) {
@@ -863,11 +871,11 @@ template <int K> __device__ __forceinline__ F2 log2_term_pair(const F2* r, const
     return f2_fma(n2, f2_mul(A[5], n2), f2_fma(n1, u1, f2_fma(n0, u0, r[0])));
 }
 
-template <typename T, int K>
+template <typename T, int K, int PER>
 __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>& b, int cur, int M, int p,
                                                 int mblock, T* s_terms) {
     // the thread's measurements: m0, m0 + blockDim.x
-    constexpr int kPer = kLikPer<T>;
+    constexpr int kPer = PER;
     const int m0 = mblock * kPer * (int)blockDim.x + threadIdx.x;
     const int G = min(b.map_n[cur][b.src[p]], prm.Gcap);
     // per Gaussian: c (-inf for a non-PD posterior), pD flag, S^-1, mean, pad -- the
@@ -1082,24 +1090,24 @@ __device__ __forceinline__ void likelihood_body(const Params& prm, const Bufs<T>
     }
 }
 
-template <typename T, int K>
-__global__ void __launch_bounds__(kLikThreads<T>) k_likelihood(__grid_constant__ const Params prm,
-                                                     __grid_constant__ const Bufs<T> b, int cur, int M) {
+template <typename T, int K, int PER>
+__global__ void __launch_bounds__(kLikThreads / PER) k_likelihood(__grid_constant__ const Params prm,
+                                                                  __grid_constant__ const Bufs<T> b, int cur, int M) {
     chain_wait();
     extern __shared__ __align__(16) unsigned char dsm_lik[];
-    likelihood_body<T, K>(prm, b, cur, M, blockIdx.x, blockIdx.y, reinterpret_cast<T*>(dsm_lik));
+    likelihood_body<T, K, PER>(prm, b, cur, M, blockIdx.x, blockIdx.y, reinterpret_cast<T*>(dsm_lik));
 }
 
 // map entry: (filter, parent, measurement block); blocks past a filter's M exit
-template <typename T, int K>
-__global__ void __launch_bounds__(kLikThreads<T>)
+template <typename T, int K, int PER>
+__global__ void __launch_bounds__(kLikThreads / PER)
     k_likelihood_batch(const __grid_constant__ SlotTable<T> tab, const FrameArgs* fas, const int4* map, int early) {
     chain_wait(early);
     extern __shared__ __align__(16) unsigned char dsm_lik[];
     const int4 e = map[blockIdx.x];
     const int M = fas[e.x].M;
-    if (e.z * kLikPer<T> * (int)blockDim.x >= M) return;
-    likelihood_body<T, K>(tab.prm[e.x], tab.b[e.x], fas[e.x].cur, M, e.y, e.z, reinterpret_cast<T*>(dsm_lik));
+    if (e.z * PER * (int)blockDim.x >= M) return;
+    likelihood_body<T, K, PER>(tab.prm[e.x], tab.b[e.x], fas[e.x].cur, M, e.y, e.z, reinterpret_cast<T*>(dsm_lik));
 }
 
 // ---------------------------------------------------------------- (d) merge
@@ -2232,7 +2240,7 @@ __global__ void __launch_bounds__(kMergeThreads, kMergeBlocks<T>)
 constexpr int kFusedThreads = 256;
 template <typename T> inline size_t fused_smem_bytes(int P, int Gcap, int Scap) {
     size_t s = cloud_fit_smem_bytes<T>(P, kFusedThreads / 32);
-    const size_t cand[3] = {prep_smem_bytes<T>(), likelihood_smem_bytes<T>(Gcap, kFusedThreads),
+    const size_t cand[3] = {prep_smem_bytes<T>(), likelihood_smem_bytes<T>(Gcap, kFusedThreads, 1),
                             merge_shared_bytes<T>(Scap, Gcap, kFusedThreads / 32)};
     for (size_t c : cand) s = c > s ? c : s;
     return s;
@@ -2245,8 +2253,8 @@ __device__ __forceinline__ void fused_parent(const Params& prm, const Bufs<T>& b
                          nullptr, nullptr, p, 0, 1, reinterpret_cast<T*>(smem));
     __syncthreads();
     prep_body<T, K>(prm, b, fa.cur, p, reinterpret_cast<T*>(smem));
-    for (int mb = 0; mb * kLikPer<T> * (int)blockDim.x < fa.M; ++mb) {
-        likelihood_body<T, K>(prm, b, fa.cur, fa.M, p, mb, reinterpret_cast<T*>(smem));
+    for (int mb = 0; mb * (int)blockDim.x < fa.M; ++mb) {
+        likelihood_body<T, K, 1>(prm, b, fa.cur, fa.M, p, mb, reinterpret_cast<T*>(smem));
         __syncthreads();
     }
     merge_body<T, K>(prm, b, fa.cur, fa.M, fa.fixed, p, prm.Scap);
