@@ -208,7 +208,8 @@ scphd_status scphd_get_launch_shapes(scphd_filter* f, int32_t* merge_threads, in
 scphd_status scphd_set_fused(scphd_filter* f, int32_t mode);
 scphd_status scphd_get_fused(scphd_filter* f, int32_t* fused);
 
-/* Cloud-fit tiling: blocks per parent (1, 2 or 4).  Each block has 4 warps and
+/* Cloud-fit tiling: blocks per parent (1, 2 or 4).  Each block has 4 warps (8 in an FP64
+ * filter or batch of fewer than 3000 parents, launched as two blocks of 4) and
  * the parent's daughter Gaussians are dealt out over the warps of all its blocks, so 2 or
  * 4 blocks per parent fill the GPU when a filter has few parents (256 blocks leave more
  * than half of the 148 SMs x 4 block slots of FP32, x 5 of FP64, idle).  By default the

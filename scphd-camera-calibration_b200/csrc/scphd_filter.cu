@@ -557,7 +557,7 @@ public:
             const int mw = merge_timed ? merge_trials % merge_candidates
                                        : (merge_chosen >= 0 ? merge_chosen : (sh.merge_threads == kMergeThreads ? 0 : 1));
             if (M > 0) ++fit_seen;
-            const int fs = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fs];
+            const int fs = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fs] * fit_unit<T>(N);
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             if (fit_specialised<T>(prm))
                 chained(k_cloud_fit<T, K, kFitP>, N * split, kFitThreads<T>, fit_smem, stream, prm, b, cur, M, fixed, pending ? 1 : 0, pending_dt, pending_frame, sample_frame[cur], zs[0], zs[1],
@@ -1711,7 +1711,7 @@ template <typename T> struct Batch final : scphd_batch {
             }
         } else {
             const bool fit_timed = split_timed();
-            const int fsi = split_now(), split = fit_splits[fsi];
+            const int fsi = split_now(), split = fit_splits[fsi] * fit_unit<T>(parents);
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             for (const Group& g : groups) {
                 if (g.fit_p)

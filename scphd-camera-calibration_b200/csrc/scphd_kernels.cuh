@@ -641,6 +641,11 @@ __device__ __forceinline__ void cloud_fit_any(const Params& prm, const Bufs<T>& 
 // threads of a cloud-fit block, and blocks an SM is to hold
 template <typename T> constexpr int kFitThreads = 32 * (sizeof(T) == 4 ? kQuadWarps : kFitWarps);
 template <typename T> constexpr int kFitBlocks = sizeof(T) == 4 ? 4 : 5;
+// Blocks of 4 warps to a unit of the split: two in FP64, where a warp takes one sample per lane,
+// unless the parents alone fill the GPU several times.  FP64, split 1, one block and two: 50
+// parents x 64 Gaussians 131, 72 us; 256 x 64 147, 112; 777 x 96 484, 418; 1500 x 160 1289,
+// 1200; 4096 x 64 1269, 1293; 4096 x 256 4919, 4882.
+template <typename T> inline int fit_unit(int parents) { return sizeof(T) == 8 && parents < 3000 ? 2 : 1; }
 template <typename T> __host__ __device__ inline size_t fit_kernel_smem_bytes(int P) {
     return sizeof(T) == 4 ? quad_fit_smem_bytes(P) : cloud_fit_smem_bytes<T>(P, kFitWarps);
 }
