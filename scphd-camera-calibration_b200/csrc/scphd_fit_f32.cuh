@@ -85,9 +85,10 @@ __device__ __forceinline__ float lg2_ftz(float x) {
 }
 
 // Box-Muller for two samples: the pair of normals Pair<float>::two gives for (wa0, wb0) in
-// the low halves and for (wa1, wb1) in the high ones.  n = -r; the root's argument
-// -2 ln u is positive for every u the clamp lets through (checked over all FP32 values in
-// [0.5, 1) on this hardware; the largest, 0.99999994, gives 8e-8).
+// the low halves and for (wa1, wb1) in the high ones.  n = -r; unlike there, nothing guards the
+// root: its argument -2 ln u is positive for every u the clamp lets through (the smallest is
+// 1.6e-8, for the largest u, 0.99999994, whose approximate logarithm is -1.2e-8 where -8.6e-8
+// is exact).  tests/cpp/normals_check.cu runs all values of [0.5, 1].
 __device__ __forceinline__ void normals_pair(uint32_t wa0, uint32_t wb0, uint32_t wa1, uint32_t wb1, F2& z0, F2& z1) {
     const F2 ua = f2_fma(pack_f32x2((float)wa0, (float)wa1), f2_dup(0x1p-32f), f2_dup(0x1p-33f));
     const F2 lg = pack_f32x2(lg2_ftz(fminf(f2_lo(ua), 0.99999994f)), lg2_ftz(fminf(f2_hi(ua), 0.99999994f)));
