@@ -432,7 +432,7 @@ def run_b200(args):
             tj = json.load(fh)
         tr = tj.get(name)
         if tr:
-            traffic = tr.get("bytes_per_launch_scaled")
+            traffic = tr.get("bytes_per_launch")
         # issue side of the cloud fit: the warp instructions per fitted Gaussian of the
         # recorded capture x the Gaussians fitted per launch, over the launch's issue slots
         # (148 SMs x 4 schedulers x the median SM clock sampled in the timed region)
@@ -442,7 +442,7 @@ def run_b200(args):
             slots = 148 * 4 * clk["sm_mhz"] * 1e6 * avg_ms / 1e3
             compute["issue"] = {"warp_instructions_per_launch": inst, "issue_slots_per_launch": slots,
                                 "frac": inst / slots,
-                                "instructions_source": "profiles/traffic.json"}
+                                "instructions_source": ti["source"]}
 
     cpu = None
     if world == 1 and not args.no_cpu_baseline:

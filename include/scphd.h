@@ -184,7 +184,7 @@ scphd_status scphd_get_counters(scphd_filter* f, int64_t counters[16]);
 
 /* Launch shapes tuned on the filter's first updates that have measurements: threads
  * per merge block (256 or 128) and the likelihood's blocks (1: one block over all of a
- * parent's measurements, 0: 128-thread blocks).  Each of the four combinations runs
+ * parent's measurements, 0: blocks of 128 measurements).  Each of the four combinations runs
  * twice, timed with events (those updates wait for the previous one), and the fastest is
  * kept.  The merge's width is timed again on grown maps, twice each on the updates with
  * measurements after the first 22 (64 threads among them for a filter of many parents).
@@ -295,9 +295,9 @@ scphd_status scphd_device_bytes(const scphd_config* cfg, int64_t* bytes);
  * use_graph != 0 the third step is captured into a CUDA graph and later steps replay it.
  * The launch shapes are tuned on six steps (not replayed) once members with half of the
  * parents have seen 16 frames; the graph is captured again after them.  Members keep the
- * shapes, and trials not finished, for the next batch they are put in.  A batched step gives each filter the same result as predict + update +
- * resample on that filter alone.  This batching has no counterpart in the reference
- * (which runs one filter per process). */
+ * shapes, and trials not finished, for the next batch they are put in.  A batched step
+ * gives each filter the same result as predict + update + resample on that filter alone.
+ * This batching has no counterpart in the reference (which runs one filter per process). */
 typedef struct scphd_frame {
     const double* u;        /* n measurements */
     const double* v;

@@ -434,8 +434,8 @@ public:
         CUDA_TRY(cudaMemsetAsync(p, 0, probe.used, stream));
         merge_smem = merge_shared_bytes<T>(prm.Scap, prm.Gcap, kMergeThreads / 32);
         fit_smem = fit_kernel_smem_bytes<T>(prm.P);
-        // with the kernel's static shared memory (20 KB at most), within 227 KB per block:
-        // every particles_per_feature up to 256 fits (FP64 at 256: 147 KB of sample rows)
+        // within 227 KB per block, every particles_per_feature up to 256 fits (at 256, rows of
+        // four warps: 75 KB in FP64)
         if (fit_smem > 200 * 1024)
             return fail(SCPHD_ERR_CAPACITY, "particles_per_feature needs " + std::to_string(fit_smem) +
                                                 " bytes of shared memory per cloud-fit block (limit 200 KB)");
@@ -560,12 +560,11 @@ public:
             const int fs = fit_timed ? fit_trials % kFitSplits : fit_chosen, split = fit_splits[fs] * fit_unit<T>(N);
             if (fit_timed) CUDA_TRY(cudaEventRecord(fit_ev[0], stream));
             if (fit_specialised<T>(prm))
-                chained(k_cloud_fit<T, K, kFitP>, N * split, kFitThreads<T>, fit_smem, stream, prm, b, cur, M, fixed, pending ? 1 : 0, pending_dt, pending_frame, sample_frame[cur], zs[0], zs[1],
-                    zs[2], split);
+                chained(k_cloud_fit<T, K, kFitP>, N * split, kFitThreads<T>, fit_smem, stream, prm, b, cur, M, fixed,
+                        pending ? 1 : 0, pending_dt, pending_frame, sample_frame[cur], zs[0], zs[1], zs[2], split);
             else
-                chained(k_cloud_fit<T, K>, N * split, kFitThreads<T>, fit_smem, stream, prm, b, cur, M, fixed, pending ? 1 : 0,
-                                                                        pending_dt, pending_frame, sample_frame[cur],
-                                                                        zs[0], zs[1], zs[2], split);
+                chained(k_cloud_fit<T, K>, N * split, kFitThreads<T>, fit_smem, stream, prm, b, cur, M, fixed,
+                        pending ? 1 : 0, pending_dt, pending_frame, sample_frame[cur], zs[0], zs[1], zs[2], split);
             LAUNCHED();
             if (fit_timed) {
                 CUDA_TRY(cudaEventRecord(fit_ev[1], stream));
@@ -642,9 +641,8 @@ public:
 
     scphd_status resample(int32_t* resampled, bool read_back) override {
         int h = stage_begin(5);
-        chained(k_resample, 1, weights_threads(prm.N), 0, stream, prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum, b.scal,
-                                                             b.flags, b.resample_idx, frame, 0, -1.0, b.counters,
-                                                             prm.N <= kGatherParents);
+        chained(k_resample, 1, weights_threads(prm.N), 0, stream, prm, b.lw, b.ext, b.ext_tmp, b.src, b.src_tmp, b.cum,
+                b.scal, b.flags, b.resample_idx, frame, 0, -1.0, b.counters, prm.N <= kGatherParents);
         LAUNCHED();
         const scphd_status gs = gather_parents();
         if (gs != SCPHD_OK) return gs;

@@ -9,11 +9,11 @@
 // both camera transforms, the motion, the moment rows) takes half the instructions, one
 // 16-byte access moves four samples of a cloud or a staged row, and the factor row and the
 // poses are read once for four samples.  Philox, the logarithm, root, sine and cosine stay
-// one per sample.  1017 instructions per fitted Gaussian at 0.55 per scheduler and cycle; one
+// one per sample.  1024 instructions per fitted Gaussian at 0.56 per scheduler and cycle; one
 // launch over 4096 parents x 256 Gaussians x 100 samples takes 1.59 ms instead of 1.98 ms.
 //
 // What bounds it now: the multiply-add pipe that runs packed operations and Philox's 64-bit
-// products (55 % busy), shared-memory data (52 %) and issue (55 %), with four warps per
+// products (54 % busy), shared-memory and L1 data (53 %) and issue (56 %), with four warps per
 // scheduler (128 registers).  Measured and not better: two samples per lane at 28 warps per
 // SM (1.90 ms: the constants are read for half as many samples, 64 % of the shared-memory
 // data path), 20 or 18 warps of 96 registers (2.05, 1.81 ms: spills that the small L1 beside

@@ -171,9 +171,9 @@ __global__ void k_predict_parents(__grid_constant__ const Params prm, double* ex
 }
 
 // ---------------------------------------------------------------- (b) cloud -> fit
-// One CTA per parent; each warp takes every eighth of the parent's daughter Gaussians,
-// a whole warp per Gaussian, after a shared tail pass per round (the sample layout
-// below).  Covers: predict_features + ps (.cu:154-178, 1144-1150),
+// A parent's daughter Gaussians are dealt out over the warps of its blocks (scphd_fit_f32.cuh
+// has the single-precision form's layout; here a whole warp takes a Gaussian, after a shared
+// tail pass per round: the sample layout below).  Covers: predict_features + ps (.cu:154-178, 1144-1150),
 // worldToDisparityKernel + computePdKernel (kernels.cu:6-47, 82-99), weight by pD
 // (.cu:1602-1609), normalizeWeightsKernel + fitGaussiansKernel (kernels.cu:996-1018,
 // 102-438) and the non-detection copy (.cu:1290-1420).
@@ -1209,14 +1209,10 @@ template <typename T> struct KalmanView {
 // single-precision keys both count as ties.  In FP32 mode the key is the weight itself.
 __device__ __forceinline__ float order_key(float w) { return w; }
 __device__ __forceinline__ float order_key(double w) { return __double2float_rn(w); }
-template <typename T> __device__ __forceinline__ bool merge_before(T wa, uint32_t ka, T wb, uint32_t kb) {
-    const float fa = order_key(wa), fb = order_key(wb);
-    return fa > fb || (fa == fb && ka < kb);
-}
 
 // A survivor's sort key: the order key's bits, made to order as the float (and the two zeros
-// as one), above the complement of the tie key, so that larger keys come first by
-// merge_before, every key is distinct and none is 0 (the padding).
+// as one), above the complement of the tie key, so that larger keys come first in the merge's
+// order, every key is distinct and none is 0 (the padding).
 __device__ __forceinline__ uint32_t float_order(float x) {
     const uint32_t bits = __float_as_uint(x + 0.0f);
     return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
@@ -1455,8 +1451,8 @@ __device__ inline void carve_merge_list(unsigned char* smem, int S, T*& s_w, uns
     ms.is_center = ms.flag + S;
 }
 
-// The filter's merge: arrays that are never live together share their bytes.  The means' area holds the sort keys before them and the new map's weights after
-// them; the u keys' holds the ranks before them, the component indices and member lists after
+// The filter's merge: arrays that are never live together share their bytes.  The means' area
+// holds the sort keys before them and the new map's weights after them; the u keys' holds the ranks before them, the component indices and member lists after
 // them; the prefilter's the output positions.  In FP32 the prefilter's u, v, d are the means'
 // (6 x S arrays), in FP64 copies.
 template <typename T> __host__ __device__ inline size_t merge_area_bytes(int S, int G) {
